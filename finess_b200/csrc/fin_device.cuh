@@ -45,21 +45,20 @@ __device__ __forceinline__ void atomic_max_nonneg(double* addr, double v)
 template <class R> __host__ __device__ __forceinline__ R Max(R a, R b) { return a > b ? a : b; }
 template <class R> __host__ __device__ __forceinline__ R Min(R a, R b) { return a < b ? a : b; }
 
-// Reciprocal by Newton-Raphson refinement of the hardware approximation
-// (PTX rcp.approx.ftz): r <- r + r(1 - x r), which squares the relative error
-// per step.  Two steps bring the FP64 approximation to within an ulp or two
-// (the plain form's parity bar is 1e-12, four orders above); FP32 uses the
-// approximation alone (~1 ulp).  x = 0 gives NaN instead of Inf; every use
-// here divides by a density, pressure or WENO weight sum, where 0 is already
-// a failed state that the non-finite check reports.
+// Reciprocal by one third-order step from the hardware approximation (PTX
+// rcp.approx.ftz): with e = 1 - x r, 1/x = r (1 + e + e^2 + ...), and the
+// series cut after e^2 cubes the approximation's relative error (about 2^-20)
+// to below an ulp in three operations (the plain form's parity bar is 1e-12,
+// four orders above); FP32 uses the approximation alone (~1 ulp).  x = 0 gives
+// NaN instead of Inf; every use here divides by a density, pressure or WENO
+// weight sum, where 0 is already a failed state that the non-finite check
+// reports.
 __device__ __forceinline__ double rcp(double x)
 {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-    double e = fma(-x, r, 1.0);
-    r = fma(r, e, r);
-    e = fma(-x, r, 1.0);
-    return fma(r, e, r);
+    const double e = fma(-x, r, 1.0);
+    return fma(r, fma(e, e, e), r);
 }
 __device__ __forceinline__ float rcp(float x)
 {
@@ -119,6 +118,33 @@ __device__ __forceinline__ float fsqrt(float x)
     asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
+
+// 1/sqrt(x) by one third-order Householder step from the hardware
+// approximation (PTX rsqrt.approx.ftz): with e = 1 - x y^2 the factor
+// (1 - e)^(-1/2) = 1 + e/2 + 3 e^2/8 + O(e^3), so the approximation's relative
+// error of about 2^-22 leaves an ulp or two in FP64 after five operations.
+// Negative x gives NaN, x = 0 gives NaN (FP64) or Inf (FP32).
+__device__ __forceinline__ double rsqrt_fast(double x)
+{
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-(x * y), y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+}
+__device__ __forceinline__ float rsqrt_fast(float x)
+{
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+// sqrt(x) for x >= 0 as x / sqrt(x); zero and subnormal x give 0 (compared on
+// the high word, which costs no FP64 instruction), Inf and NaN give NaN.
+__device__ __forceinline__ double sqrt_fast(double x)
+{
+    const double s = x * rsqrt_fast(x);
+    return __double2hiint(x) < 0x00100000 ? 0.0 : s;
+}
+__device__ __forceinline__ float sqrt_fast(float x) { return fsqrt(x); }
 
 // ---------------------------------------------------------------------------
 // Euler callbacks (apps/2d/euler/lib).  Component order inside a face is the
@@ -231,6 +257,58 @@ struct Euler {
         w1 = (r.e1 * v[0] + e.u1 * v[1] + e.u2 * v[2] + e.u3 * v[3] - v[4]) * e.inv_d2;
     }
 
+    // The face's eigen data in the form the stage kernels project with.  With
+    // h = H - |u|^2/2 = c^2/(gamma-1), k = 1/(2 h) and hc = 1/(2 c) the rows of
+    // ProjectLeftEig.cpp:47-66 share two combinations,
+    //   s = v4 - u1 v1 - u2 v2 - u3 v3 + |u|^2/2 v0,   m = v1 - u1 v0:
+    //   W0 = k s - hc m,  W4 = k s + hc m,  W1 = v0 - 2 k s,
+    //   W2 = v2 - u2 v0,  W3 = v3 - u3 v0
+    // (11 operations a vector against 19 for the rows written out), and one
+    // reciprocal square root gives c, k and hc.  The right projection
+    // (ProjectRightEig.cpp:46-62) shares its sums the same way.
+    template <class R>
+    struct Face { R u1, u2, u3, hu2, c, h, k, hc, ir; };
+
+    template <class R>
+    __device__ __forceinline__ static Face<R> face(R gamma, const R* Qn)
+    {
+        Face<R> e;
+        e.ir = rcp(Qn[0]);
+        e.u1 = Qn[1] * e.ir;
+        e.u2 = Qn[2] * e.ir;
+        e.u3 = Qn[3] * e.ir;
+        e.hu2 = R(0.5) * (e.u1 * e.u1 + e.u2 * e.u2 + e.u3 * e.u3);
+        const R press = (gamma - R(1)) * (Qn[4] - Qn[0] * e.hu2);
+        const R c2 = gamma * press * e.ir;
+        const R ic = rsqrt_fast(c2);   // NaN for a negative pressure, as ProjectLeftEig.cpp:43's sqrt
+        e.c = c2 * ic;
+        e.h = (Qn[4] + press) * e.ir - e.hu2;
+        e.hc = R(0.5) * ic;
+        e.k = (gamma - R(1)) * ic * e.hc;
+        return e;
+    }
+    // Rows 0, 1 and 4 of the left projection of one vector.
+    template <class R>
+    __device__ __forceinline__ static void left014(const Face<R>& e, const R* v, R& w0, R& w1, R& w4)
+    {
+        const R ks = e.k * (e.hu2 * v[0] + (v[4] - e.u1 * v[1] - e.u2 * v[2] - e.u3 * v[3]));
+        const R m = v[1] - e.u1 * v[0];
+        w0 = ks - e.hc * m;
+        w4 = ks + e.hc * m;
+        w1 = v[0] - R(2) * ks;
+    }
+    // Right projection of the five amplitudes.
+    template <class R>
+    __device__ __forceinline__ static void right(const Face<R>& e, const R* g, R* f)
+    {
+        const R s = g[0] + g[4], cd = e.c * (g[4] - g[0]);
+        f[0] = s + g[1];
+        f[1] = e.u1 * f[0] + cd;
+        f[2] = e.u2 * f[0] + g[2];
+        f[3] = e.u3 * f[0] + g[3];
+        f[4] = e.h * s + e.hu2 * f[0] + e.u1 * cd + e.u2 * g[2] + e.u3 * g[3];
+    }
+
     // ProjectLeftEig.cpp:47-66 for one point (normal frame in and out).
     template <class R>
     __device__ __forceinline__ static void left(const Eig<R>& e, const R* Q, R* W)
@@ -327,44 +405,60 @@ __device__ __forceinline__ void weno5_parts(const R* u, R& b0, R& b1, R& b2, R& 
     c2 = (R(1) / R(3)) * ui + (R(5) / R(6)) * uip1 - (R(1) / R(6)) * uip2;
 }
 
+// On the four first differences d1 .. d4 of the stencil: with t_k the second
+// differences and s_k the first-derivative forms, 4 beta_k = 13/3 t_k^2 +
+// s_k^2, and candidate k is u_i + p_k / 6 with p_0 = 5 d2 - 2 d1, p_1 = d2 +
+// 2 d3, p_2 = 4 d3 - d4, so the value at i+1/2 is u_i + c / 6 with
+//   c = sum w_k p_k / sum w_k
+// (what this function returns) and, for power 2, w_k = g_k x_j^2 x_l^2 (JS) or
+// g_k (x_k^2 + T) x_j^2 x_l^2 (Z), x_k = 4 (eps + beta_k), T = (x_0 - x_2)^2.
+// 42 (Z) or 36 (JS) operations after the differences, against 63 and 55 for
+// the candidates and indicators written on the point values, and the
+// rounding error scales with the differences.
+template <class R, int VER, bool P2>
+__device__ __forceinline__ R weno5_diff(R d1, R d2, R d3, R d4, R eps4, R pw)
+{
+    const R s0 = R(3) * d2 - d1, s2 = d4 - R(3) * d3;
+    const R p0 = R(2) * s0 - d2, p1 = d2 + R(2) * d3, p2 = d3 - s2;
+    if constexpr (VER == FIN_WENO_FD) {
+        return R(0.1) * p0 + (R(0.6) * p1 + R(0.3) * p2);
+    } else {
+        const R t0 = d2 - d1, t1 = d3 - d2, t2 = d4 - d3, s1 = d2 + d3;
+        const R K = R(13) / R(3);
+        const R x0 = s0 * s0 + ((K * t0) * t0 + eps4);
+        const R x1 = s1 * s1 + ((K * t1) * t1 + eps4);
+        const R x2 = s2 * s2 + ((K * t2) * t2 + eps4);
+        R w0, w1, w2;
+        if constexpr (P2) {
+            R X0 = x0 * x0, X1 = x1 * x1, X2 = x2 * x2;
+            R T = R(0);
+            if (VER == FIN_WENO_Z) { const R tau = x0 - x2; T = tau * tau; }
+            if (sizeof(R) == 4) {
+                const R s = rcp(Max(X0, Max(X1, X2)));
+                X0 *= s; X1 *= s; X2 *= s; T *= s;
+            }
+            w0 = X1 * X2; w1 = X0 * X2; w2 = X0 * X1;
+            if (VER == FIN_WENO_Z) {
+                const R P = X0 * w0;
+                w0 = T * w0 + P; w1 = T * w1 + P; w2 = T * w2 + P;
+            }
+        } else if (VER == FIN_WENO_JS) {
+            w0 = pow(R(0.25) * x0, -pw); w1 = pow(R(0.25) * x1, -pw); w2 = pow(R(0.25) * x2, -pw);
+        } else {
+            const R tau = fabs(x0 - x2);
+            w0 = R(1) + pow(tau / x0, pw); w1 = R(1) + pow(tau / x1, pw); w2 = R(1) + pow(tau / x2, pw);
+        }
+        w1 = R(6) * w1;
+        w2 = R(3) * w2;
+        return (w0 * p0 + w1 * p1 + w2 * p2) * rcp(w0 + w1 + w2);
+    }
+}
+
 template <class R, int VER, bool P2>
 __device__ __forceinline__ R weno5(const R* u, R eps, R pw)
 {
-    R b0, b1, b2, c0, c1, c2;
-    weno5_parts(u, b0, b1, b2, c0, c1, c2);
-    if (VER == FIN_WENO_FD) return R(0.1) * c0 + R(0.6) * c1 + R(0.3) * c2;
-    R w0, w1, w2;
-    if (P2) {
-        const R d0 = eps + b0, d1 = eps + b1, d2 = eps + b2;
-        R D0 = d0 * d0, D1 = d1 * d1, D2 = d2 * d2;
-        R T = R(0);
-        if (VER == FIN_WENO_Z) { const R tau = fabs(b0 - b2); T = tau * tau; }
-        if (sizeof(R) == 4) {
-            const R s = rcp(Max(D0, Max(D1, D2)));
-            D0 *= s; D1 *= s; D2 *= s; T *= s;
-        }
-        if (VER == FIN_WENO_JS) {
-            w0 = R(0.1) * (D1 * D2);
-            w1 = R(0.6) * (D0 * D2);
-            w2 = R(0.3) * (D0 * D1);
-        } else {
-            w0 = R(0.1) * ((D0 + T) * (D1 * D2));
-            w1 = R(0.6) * ((D1 + T) * (D0 * D2));
-            w2 = R(0.3) * ((D2 + T) * (D0 * D1));
-        }
-    } else {
-        if (VER == FIN_WENO_JS) {
-            w0 = R(0.1) * pow(eps + b0, -pw);
-            w1 = R(0.6) * pow(eps + b1, -pw);
-            w2 = R(0.3) * pow(eps + b2, -pw);
-        } else {
-            const R tau = fabs(b0 - b2);
-            w0 = R(0.1) * (R(1) + pow(tau / (eps + b0), pw));
-            w1 = R(0.6) * (R(1) + pow(tau / (eps + b1), pw));
-            w2 = R(0.3) * (R(1) + pow(tau / (eps + b2), pw));
-        }
-    }
-    return (w0 * c0 + w1 * c1 + w2 * c2) * rcp(w0 + w1 + w2);
+    return u[2] + (R(1) / R(6)) * weno5_diff<R, VER, P2>(u[1] - u[0], u[2] - u[1], u[3] - u[2], u[4] - u[3],
+                                                         R(4) * eps, pw);
 }
 
 // The two WENO5 reconstructions of a face's split (u = gp, the points of

@@ -23,15 +23,32 @@
 //   gs  [M][TI][TJ+6]     y flux g at the y-stencil cells
 //   Fh  [M][TI+1][TJ]     x-face numerical fluxes
 //   Gh  [M][TI][TJ+1]     y-face numerical fluxes
-// Phases: load (coalesced along j) -> flux per cell (FluxFunc once per cell,
+//   opnd [M][TI][TJ]      the stage operand that is not q_in (FP64)
+// Phases: load (coalesced along j) and flux per cell (FluxFunc once per cell,
 // not six times per face as the reference does) -> one thread per face, x
-// and y faces in one work list (projection, LLF split, two WENO5, back
-// projection, all in registers) -> per cell flux difference + RK update +
-// next-stage wave speed -> block max -> one atomicMax per block.
+// faces then y faces (projection, LLF split, two WENO5, back projection, all
+// in registers) -> per cell flux difference + RK update + next-stage wave
+// speed -> block max -> one atomicMax per block.
+//
+// What bounds it: the FP64 form is bound by the FP64 pipe and by the latency
+// of dependent FP64 operations at 16 warps per SM (128 registers), so what
+// counts is instructions per face and registers.  Measured, SSP-RK3 step at
+// 4096^2 (three launches, ms): 10.54 with candidates and smoothness
+// indicators on point values, projection rows written out and one face body
+// for both directions; 8.75 with the difference form (weno5_diff), the shared
+// projection sums (Euler::Face) and the upwind part of the flux parked in its
+// slot; 7.58 with one body per direction (constant stencil offsets: integer
+// multiply-adds and moves fell from 17 to 4 % of the instructions, spills
+// from 180 to 70 bytes), load and flux phases in one, the stage operand
+// copied behind the face phase (q_in's own values taken from shared memory)
+// and the warp maxima by two reduce instructions each.  The FP64 pipe is 61 %
+// busy (52 % before).  The same body changes took the FP32 form's step from
+// 1.69 to 1.48 ms (two steps of 4001 x 515).
 #pragma once
 #include "fin_device.cuh"
 #include "fin_tc.cuh"
 #include "fin_weno_face.cuh"
+#include <type_traits>
 
 namespace fin {
 
@@ -120,9 +137,15 @@ struct TileCfg {
     __host__ __device__ static constexpr bool XROW8() { return sizeof(R) == 4 && TI == 15 && TJ == 16; }
     template <class R>
     __host__ __device__ static constexpr int FSJ() { return XROW8<R>() ? TJ + 2 : TJ; }
-    // byte offset of the reduction scratch (after the arrays, 16-B aligned)
+    // byte offsets of the staged stage operand (FP64) and of the reduction
+    // scratch (after the arrays, 16-B aligned)
     template <class R>
     __host__ __device__ static constexpr size_t red_offset()
+    {
+        return opnd_offset<R>() + (sizeof(R) == 8 ? size_t(MEQN) * TI * TJ * 8 : 0);
+    }
+    template <class R>
+    __host__ __device__ static constexpr size_t opnd_offset()
     {
         return (sizeof(R) * (size_t(MEQN) * (size_t(RI) * RJ + size_t(RI) * FSJ<R>() + size_t(TI) * RJ +
                                              size_t(TI + 1) * TJ + size_t(TI) * (TJ + 1)) +
@@ -219,12 +242,6 @@ __device__ __forceinline__ R linear_face(const R* f, int fstr, const R* q, int q
 #define FIN_MINB_F32 3
 #endif
 template <class R> struct MinBlocks { static constexpr int value = FIN_MINB_F64; };
-// FP64 face body: fields 0, 4 and 1 in one sweep of the stencil (1: one
-// load and split of each stencil point instead of two; measured 4 % faster
-// on B200 at 4096^2) or the three passes of the register-lean form (0).
-#ifndef FIN_F64_MERGE
-#define FIN_F64_MERGE 1
-#endif
 template <> struct MinBlocks<float> { static constexpr int value = FIN_MINB_F32; };
 
 // Scalar parameters read from kernel-parameter space where they are used
@@ -250,42 +267,248 @@ template <> struct Par<float> {
 __device__ __forceinline__ void fence(double& x) { asm volatile("" : "+d"(x)); }
 __device__ __forceinline__ void fence(float& x) { asm volatile("" : "+f"(x)); }
 template <class R>
-__device__ __forceinline__ void fence5(R* u)
+__device__ __forceinline__ void fence4(R* u)
 {
 #pragma unroll
-    for (int k = 0; k < 5; k++) fence(u[k]);
+    for (int k = 0; k < 4; k++) fence(u[k]);
 }
 
-// gp and gm reconstructions of one characteristic field, fenced as a unit.
+// Corrections (weno5_diff) of gp and gm of one characteristic field from the
+// differences of their stencils, fenced as a unit.
 template <class R, int VER, bool P2>
-__device__ __forceinline__ R weno_pair(R* up, R* um, R eps, R pw)
+__device__ __forceinline__ R weno_pair(R* dp, R* dm, R eps4, R pw)
 {
-    fence5(up);
-    fence5(um);
-    R g;
-    if constexpr (sizeof(R) == 4 && (P2 || VER == FIN_WENO_FD)) g = weno5_pair_x2<VER>(up, um, eps);   // f32x2 pairs
-    else g = weno5<R, VER, P2>(up, eps, pw) + weno5<R, VER, P2>(um, eps, pw);
+    fence4(dp);
+    fence4(dm);
+    R g = weno5_diff<R, VER, P2>(dp[0], dp[1], dp[2], dp[3], eps4, pw) +
+          weno5_diff<R, VER, P2>(dm[0], dm[1], dm[2], dm[3], eps4, pw);
     fence(g);
     return g;
 }
 
-// Right projection (ProjectRightEig.cpp:46-62) of one characteristic field k
-// with amplitude gk, added into the face flux f[0..4] (normal frame).  The
-// projection is linear, so the face flux is accumulated field by field.
-template <class R>
-__device__ __forceinline__ void right_add(const typename Euler::Eig<R>& e, int k, R gk, R* f)
+// Max over a warp of non-negative doubles, as the maximum of their high words
+// and then of the low words that go with it (two warp-reduce instructions
+// instead of five rounds of two shuffles, a compare and two selects).
+__device__ __forceinline__ double warp_max_nonneg(double v)
 {
-    if (k == 0) {
-        f[0] += gk; f[1] += (e.u1 - e.c) * gk; f[2] += e.u2 * gk; f[3] += e.u3 * gk; f[4] += (e.H - e.u1 * e.c) * gk;
-    } else if (k == 4) {
-        f[0] += gk; f[1] += (e.u1 + e.c) * gk; f[2] += e.u2 * gk; f[3] += e.u3 * gk; f[4] += (e.H + e.u1 * e.c) * gk;
-    } else if (k == 1) {
-        f[0] += gk; f[1] += e.u1 * gk; f[2] += e.u2 * gk; f[3] += e.u3 * gk; f[4] += e.hu2 * gk;
-    } else if (k == 2) {
-        f[2] += gk; f[4] += e.u2 * gk;
-    } else {
-        f[3] += gk; f[4] += e.u3 * gk;
+    const unsigned hi = unsigned(__double2hiint(v));
+    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? unsigned(__double2loint(v)) : 0u);
+    return __hiloint2double(int(mh), int(ml));
+}
+
+// Shared-memory arrays of a stage tile.
+template <class R, class Cfg>
+struct StageSmem {
+    static constexpr int PQ = Cfg::RI * Cfg::RJ, FS = Cfg::template FSJ<R>();
+    R* prim;   // [4][RI][RJ]   u, v, p, c
+    R* qs;     // [M][RI][RJ]
+    R* fs;     // [M][RI][FS]   0.5 * f
+    R* gs;     // [M][TI][RJ]   0.5 * g
+    R* Fh;     // [M][TI+1][TJ]
+    R* Gh;     // [M][TI][TJ+1]
+    double* opnd;   // [M][TI*TJ] the stage operand that is not q_in (FP64)
+    double* red;
+    __device__ __forceinline__ explicit StageSmem(unsigned char* raw)
+    {
+        prim = reinterpret_cast<R*>(raw);
+        qs = prim + Cfg::NPRIM * PQ;
+        fs = qs + MEQN * PQ;
+        gs = fs + MEQN * Cfg::RI * FS;
+        Fh = gs + MEQN * Cfg::TI * Cfg::RJ;
+        Gh = Fh + MEQN * (Cfg::TI + 1) * Cfg::TJ;
+        opnd = reinterpret_cast<double*>(raw + Cfg::template opnd_offset<R>());
+        red = reinterpret_cast<double*>(raw + Cfg::template red_offset<R>());
     }
+};
+
+// Flux of face k of direction x (ISX: between rows fi-1 and fi of the tile)
+// or y (between columns fj-1 and fj), in registers; the direction is a
+// template parameter, so every stencil address is a constant offset.  Returns
+// the face's LLF speed and whether it enters GetCFL's maximum in *in_cfl.
+template <class R, int VER, bool P2, class Cfg, bool FG, bool ISX>
+__device__ __forceinline__ R stage_face(const StageArgs& a, const StageSmem<R, Cfg>& S, int w, int i0, int j0, R ag,
+                                        bool& neg, bool& in_cfl)
+{
+    constexpr int TI = Cfg::TI, TJ = Cfg::TJ, H = Cfg::H, RI = Cfg::RI, RJ = Cfg::RJ;
+    constexpr int PQ = RI * RJ, FS = Cfg::template FSJ<R>();
+    constexpr int CN = ISX ? 1 : 2, CT = ISX ? 2 : 1;   // normal / tangential momentum
+    constexpr int QSTR = ISX ? RJ : 1, FSTR = ISX ? FS : 1, FP = ISX ? RI * FS : TI * RJ;
+    constexpr int OP = ISX ? (TI + 1) * TJ : TI * (TJ + 1);
+#define gamma (Par<R>::gamma(a))
+#define eps (Par<R>::eps(a))
+#define pw (Par<R>::pw(a))
+    int fi, fj;
+    if (ISX) {
+        if constexpr (Cfg::template XROW8<R>()) {
+            fi = (w >> 5) + ((w >> 1) & 8); fj = w & 15;   // half-warps on rows r and r + 8
+        } else {
+            fi = w / TJ; fj = w - fi * TJ;
+        }
+    } else {
+        // taken by rows of TJ, then the last column, so a half-warp reads one
+        // row of the staged tile (FP32: half-warps on rows r and r + 8; the
+        // last warp takes row 7 and the last column)
+        if constexpr (Cfg::template XROW8<R>()) {
+            const int wv = w >> 5, ln = w & 31;
+            if (wv < 7) { fi = wv + (ln & 16 ? 8 : 0); fj = ln & 15; }
+            else if (ln < 16) { fi = 7; fj = ln; }
+            else { fi = ln - 16; fj = TJ; }
+        } else {
+            fi = w < TI * TJ ? w / TJ : w - TI * TJ;
+            fj = w < TI * TJ ? w - fi * TJ : TJ;
+        }
+    }
+    const R* const qb = S.qs + (H + fi) * RJ + (H + fj);
+    const R* const pb = S.prim + (H + fi) * RJ + (H + fj);
+    const R* const fb = ISX ? S.fs + (H + fi) * FS + fj : S.gs + fi * RJ + (H + fj);
+    R* const out = ISX ? S.Fh + fi * TJ + fj : S.Gh + fi * (TJ + 1) + fj;
+    // Face average (ConstructL.cpp:72-77) in the normal frame.
+    R Qa[MEQN];
+    Qa[0] = R(0.5) * (qb[0] + qb[-QSTR]);
+    Qa[1] = R(0.5) * (qb[CN * PQ] + qb[CN * PQ - QSTR]);
+    Qa[2] = R(0.5) * (qb[CT * PQ] + qb[CT * PQ - QSTR]);
+    Qa[3] = R(0.5) * (qb[3 * PQ] + qb[3 * PQ - QSTR]);
+    Qa[4] = R(0.5) * (qb[4 * PQ] + qb[4 * PQ - QSTR]);
+    constexpr bool X2 = sizeof(R) == 4 && (P2 || VER == FIN_WENO_FD);   // FP32: f32x2 pairs
+    typename std::conditional<X2, Euler::Eig<R>, Euler::Face<R>>::type ev;
+    R ir;
+    if constexpr (X2) { ev = Euler::eig(gamma, Qa); ir = rcp(Qa[0]); }
+    else { ev = Euler::face(gamma, Qa); ir = ev.ir; }
+    // SetWaveSpd.cpp:39-68 from the two cells' u_n, p, c (nmag = 1) and
+    // the LLF alpha of ConstructL.cpp:172-174.
+    R alpha;
+    {
+        constexpr int UN = ISX ? 0 : 1;
+        const R unl = pb[UN * PQ - QSTR], unr = pb[UN * PQ];
+        const R pl = pb[2 * PQ - QSTR], pr = pb[2 * PQ];
+        const R cl = pb[3 * PQ - QSTR], cr = pb[3 * PQ];
+        const R ua = R(0.5) * (unl + unr);
+        const R pa = R(0.5) * (pl + pr);
+        const R ca = sqrt_fast(fabs(gamma * pa * ir));
+        if (pa < R(0) || Qa[0] < R(0)) neg = true;
+        const R s1 = Min(unl - cl, ua - ca);
+        const R s2 = Max(unr + cr, ua + ca);
+        alpha = Max(ag, Max(fabs(s1), fabs(s2)));
+    }
+    // GetCFL's Max skips NaN entries (Max(NaN, c) = c), so only finite face
+    // speeds enter the CFL maximum.
+    const int gi = i0 + fi, gj = j0 + fj;
+    in_cfl = gi < a.mx && gj < a.my && !(FG && a.flux_only && gi == 0 && gj == 0);
+    {
+        double* const fa = ISX ? a.face_alpha_x : a.face_alpha_y;
+        if (fa && gi < a.mx + (ISX ? 1 : 0) && gj < a.my + (ISX ? 0 : 1))
+            fa[size_t(gi) * (a.my + (ISX ? 0 : 1)) + gj] = double(alpha);
+    }
+    // gp = 0.5 (L f + l_alpha L q) = L (0.5 f + 0.5 l_alpha q), points
+    // 0..4; gm the same with -l_alpha, points 5..1 (ConstructL.cpp:179-185).
+    const R lah = R(0.5) * Par<R>::ascale(a) * alpha;
+    R fh[MEQN];
+    if constexpr (X2) {
+        // the split pairs and the paired reconstructions of weno_char_flux_x2
+        auto pt = [&](int s, float* q, float* f) {
+            const int oq = (s - 3) * QSTR, of = (s - 3) * FSTR;
+            q[0] = qb[oq]; q[1] = qb[CN * PQ + oq]; q[2] = qb[CT * PQ + oq]; q[3] = qb[3 * PQ + oq];
+            q[4] = qb[4 * PQ + oq];
+            f[0] = fb[of]; f[1] = fb[CN * FP + of]; f[2] = fb[CT * FP + of]; f[3] = fb[3 * FP + of];
+            f[4] = fb[4 * FP + of];
+        };
+        weno_char_flux_x2<VER>(ev, lah, pt, eps, fh);
+    } else {
+        // The reconstructed split values are their upwind points plus
+        // corrections (weno5_diff), and R L = I, so the face flux is
+        //   (v+ of the left cell + v- of the right cell) + R corr / 6:
+        // the first term in conserved variables, parked in the flux slot
+        // (it would hold ten registers through the sweeps), the second
+        // from differences of the projected points.  Fields 0, 4 and 1 in
+        // one sweep of the stencil, then 2 and 3 (all five at once want
+        // more registers than two CTAs per SM leave).
+#pragma unroll
+        for (int m = 0; m < MEQN; m++)
+            out[m * OP] = (fb[m * FP - FSTR] + fb[m * FP]) + lah * (qb[m * PQ - QSTR] - qb[m * PQ]);
+        R g[MEQN];
+        const R eps4 = R(4) * eps;
+        {
+            R p0[4], p4[4], m0[4], m4[4], p1[4], m1[4];
+            R cp0, cp1, cp4, cm0, cm1, cm4;   // the previous point's values
+#pragma unroll
+            for (int s = 0; s < 6; s++) {
+                // keep the compiler from hoisting every stencil point's loads
+                // ahead of the arithmetic
+                asm volatile("" ::: "memory");
+                const int oq = (s - 3) * QSTR, of = (s - 3) * FSTR;
+                const R q0 = qb[oq], qn = qb[CN * PQ + oq], qt = qb[CT * PQ + oq], qw = qb[3 * PQ + oq],
+                        qe = qb[4 * PQ + oq];
+                const R f0 = fb[of], fn = fb[CN * FP + of], ft = fb[CT * FP + of], fw = fb[3 * FP + of],
+                        fe = fb[4 * FP + of];
+                R w0, w1, w4;
+                if (s < 5) {
+                    const R v[MEQN] = {f0 + lah * q0, fn + lah * qn, ft + lah * qt, fw + lah * qw, fe + lah * qe};
+                    Euler::left014(ev, v, w0, w1, w4);
+                    if (s > 0) { p0[s - 1] = w0 - cp0; p1[s - 1] = w1 - cp1; p4[s - 1] = w4 - cp4; }
+                    cp0 = w0; cp1 = w1; cp4 = w4;
+                }
+                if (s > 0) {
+                    const R v[MEQN] = {f0 - lah * q0, fn - lah * qn, ft - lah * qt, fw - lah * qw, fe - lah * qe};
+                    Euler::left014(ev, v, w0, w1, w4);
+                    if (s > 1) { m0[5 - s] = cm0 - w0; m1[5 - s] = cm1 - w1; m4[5 - s] = cm4 - w4; }
+                    cm0 = w0; cm1 = w1; cm4 = w4;
+                }
+            }
+            g[0] = weno_pair<R, VER, P2>(p0, m0, eps4, pw);
+            g[4] = weno_pair<R, VER, P2>(p4, m4, eps4, pw);
+            g[1] = weno_pair<R, VER, P2>(p1, m1, eps4, pw);
+        }
+        {
+            // fields 2 and 3 (rows v_t - u2 v0 and v_w - u3 v0)
+            R p2[4], p3[4], m2[4], m3[4];
+            R cp2, cp3, cm2, cm3;
+#pragma unroll
+            for (int s = 0; s < 6; s++) {
+                asm volatile("" ::: "memory");
+                const int oq = (s - 3) * QSTR, of = (s - 3) * FSTR;
+                const R q0 = qb[oq], qt = qb[CT * PQ + oq], qw = qb[3 * PQ + oq];
+                const R f0 = fb[of], ft = fb[CT * FP + of], fw = fb[3 * FP + of];
+                if (s < 5) {
+                    const R v0 = f0 + lah * q0;
+                    const R w2 = (ft + lah * qt) - ev.u2 * v0, w3 = (fw + lah * qw) - ev.u3 * v0;
+                    if (s > 0) { p2[s - 1] = w2 - cp2; p3[s - 1] = w3 - cp3; }
+                    cp2 = w2; cp3 = w3;
+                }
+                if (s > 0) {
+                    const R v0 = f0 - lah * q0;
+                    const R w2 = (ft - lah * qt) - ev.u2 * v0, w3 = (fw - lah * qw) - ev.u3 * v0;
+                    if (s > 1) { m2[5 - s] = cm2 - w2; m3[5 - s] = cm3 - w3; }
+                    cm2 = w2; cm3 = w3;
+                }
+            }
+            g[2] = weno_pair<R, VER, P2>(p2, m2, eps4, pw);
+            g[3] = weno_pair<R, VER, P2>(p3, m3, eps4, pw);
+        }
+        Euler::right(ev, g, fh);
+        const R s6 = R(1) / R(6);
+        fh[0] = s6 * fh[0] + out[0];
+        fh[1] = s6 * fh[1] + out[CN * OP];
+        fh[2] = s6 * fh[2] + out[CT * OP];
+        fh[3] = s6 * fh[3] + out[3 * OP];
+        fh[4] = s6 * fh[4] + out[4 * OP];
+    }
+    // Back to (rho, rho u, rho v, rho w, E) and store.
+    const R o[MEQN] = {fh[0], fh[CN], fh[CT], fh[3], fh[4]};
+#pragma unroll
+    for (int m = 0; m < MEQN; m++) out[m * OP] = o[m];
+    if (FG) {
+        double* const fo = ISX ? a.flux_x : a.flux_y;
+        const int ni = a.mx + (ISX ? 1 : 0), nj = a.my + (ISX ? 0 : 1);
+        if (fo && gi < ni && gj < nj) {
+#pragma unroll
+            for (int m = 0; m < MEQN; m++) fo[(size_t(m) * ni + gi) * nj + gj] = double(o[m]);
+        }
+    }
+#undef gamma
+#undef eps
+#undef pw
+    return alpha;
 }
 
 // One tile (rows i0 .., columns j0 ..) of a stage; the whole CTA takes part.
@@ -295,401 +518,145 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const int i0, con
     constexpr int TI = Cfg::TI, TJ = Cfg::TJ, NT = Cfg::NT, H = Cfg::H;
     constexpr int RI = Cfg::RI, RJ = Cfg::RJ;
     constexpr int PQ = RI * RJ;                    // plane size of qs and prim
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    R* prim = reinterpret_cast<R*>(smem_raw);      // [4][RI][RJ]   u, v, p, c
-    R* qs = prim + Cfg::NPRIM * PQ;                // [M][RI][RJ]
     constexpr int FS = Cfg::template FSJ<R>();
-    R* fs = qs + MEQN * PQ;                        // [M][RI][FS]   0.5 * f
-    R* gs = fs + MEQN * RI * FS;                   // [M][TI][RJ]   0.5 * g
-    R* Fh = gs + MEQN * TI * RJ;                   // [M][TI+1][TJ]
-    R* Gh = Fh + MEQN * (TI + 1) * TJ;             // [M][TI][TJ+1]
-    double* red = reinterpret_cast<double*>(smem_raw + Cfg::template red_offset<R>());
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    const StageSmem<R, Cfg> S(smem_raw);
 
     const int tid = threadIdx.x;
     const int mx = a.mx, my = a.my;
-#define gamma (Par<R>::gamma(a))
+    // The stage operand other than q_in (FP64: copied to shared memory behind
+    // the face phase; q_in's own interior values are already there).
+    const double* const ext = (a.A && a.A != a.qin) ? a.A : ((a.B && a.B != a.qin) ? a.B : nullptr);
+    constexpr bool OPND = sizeof(R) == 8;
+    if (OPND && ext && !(FG && a.flux_only)) {
+        for (int c = tid; c < TI * TJ; c += NT) {
+            const int ci = c / TJ, gi = i0 + ci, gj = j0 + (c - ci * TJ);
+            if (gi < mx && gj < my) {
+                const double* src = ext + size_t(gi) * my + gj;
+                const unsigned dst = unsigned(__cvta_generic_to_shared(S.opnd + c));
+#pragma unroll
+                for (int m = 0; m < MEQN; m++)
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + m * TI * TJ * 8), "l"(src + m * a.plane));
+            }
+        }
+    }
 
-    // ---- phase 0: load the tile + halo, boundary conditions by remap ----
-    // FP64: all of a thread's loads are issued before its stores (one memory
-    // round trip per tile, not one per pass over the region; 1-3 % faster at
-    // 2 CTAs per SM).  FP32 (3 CTAs per SM, whose register budget it tightens)
-    // keeps one pass at a time.
-    if constexpr (sizeof(R) == 4) {
-        for (int e = tid; e < PQ; e += NT) {
-            const int ii = e / RJ, jj = e - ii * RJ;
-            const bool xin = ii >= H && ii < H + TI, yin = jj >= H && jj < H + TJ;
-            if (!xin && !yin) continue;
+    // ---- phase 1: load the tile + halo, boundary conditions by remap, and per
+    // cell of the cross region FluxFunc (FluxFunc.cpp:19-42, once per cell
+    // instead of once per stencil point of every face), halved for the LLF
+    // split, and the cell's u, v, p, c for SetWaveSpd.cpp:24-50 ----
+    // FP64: all of a thread's loads are issued before its arithmetic (one
+    // memory round trip per tile, not one per pass over the region).  FP32
+    // (3 CTAs per SM, whose register budget it tightens) keeps one pass at a
+    // time.
+    {
+        constexpr int NIT = (PQ + NT - 1) / NT;
+        constexpr int NV = sizeof(R) == 8 ? NIT : 1;
+        auto in_cross = [&](int e, int& ii, int& jj) {
+            ii = e / RJ;
+            jj = e - ii * RJ;
+            return e < PQ && ((ii >= H && ii < H + TI) || (jj >= H && jj < H + TJ));
+        };
+        auto load = [&](int e, R* v) {
+            int ii, jj;
+            if (!in_cross(e, ii, jj)) return;
             const int gi = bc_remap(i0 + ii - H, mx, a.bc[0], a.bc[1]);
             const int gj = bc_remap(j0 + jj - H, my, a.bc[2], a.bc[3]);
             const size_t g = size_t(gi) * my + gj;
 #pragma unroll
-            for (int m = 0; m < MEQN; m++) qs[m * PQ + e] = R(__ldg(a.qin + m * a.plane + g));
-        }
-        __syncthreads();
-    } else {
-        constexpr int NIT = (PQ + NT - 1) / NT;
-        double v[NIT][MEQN];
-#pragma unroll
-        for (int it = 0; it < NIT; it++) {
-            const int e = tid + it * NT;
-            const int ii = e / RJ, jj = e - ii * RJ;
+            for (int m = 0; m < MEQN; m++) v[m] = R(__ldg(a.qin + m * a.plane + g));
+        };
+        auto cell = [&](int e, const R* v) {
+            int ii, jj;
+            if (!in_cross(e, ii, jj)) return;
             const bool xin = ii >= H && ii < H + TI, yin = jj >= H && jj < H + TJ;
-            if (e < PQ && (xin || yin)) {
-                const int gi = bc_remap(i0 + ii - H, mx, a.bc[0], a.bc[1]);
-                const int gj = bc_remap(j0 + jj - H, my, a.bc[2], a.bc[3]);
-                const size_t g = size_t(gi) * my + gj;
+            const R gam = Par<R>::gamma(a);
 #pragma unroll
-                for (int m = 0; m < MEQN; m++) v[it][m] = __ldg(a.qin + m * a.plane + g);
+            for (int m = 0; m < MEQN; m++) S.qs[m * PQ + e] = v[m];
+            const R rho = v[0], m1 = v[1], m2 = v[2], m3 = v[3], en = v[4];
+            const R ir = rcp(rho);
+            const R u1 = m1 * ir, u2 = m2 * ir, u3 = m3 * ir;
+            const R press = (gam - R(1)) * (en - R(0.5) * rho * (u1 * u1 + u2 * u2 + u3 * u3));
+            S.prim[e] = u1;
+            S.prim[PQ + e] = u2;
+            S.prim[2 * PQ + e] = press;
+            S.prim[3 * PQ + e] = sqrt_fast(fabs(gam * press * ir));
+            if (FG) {
+                // 0.5 * F, 0.5 * G of the integrated-flux kernel, unremapped: it
+                // covers the 3-cell ghost frame; cells of a partial tile beyond it
+                // only feed discarded faces, so their index is clamped.
+                int ci = i0 + ii - H, cj = j0 + jj - H;
+                ci = ci < -3 ? -3 : (ci > mx + 2 ? mx + 2 : ci);
+                cj = cj < -3 ? -3 : (cj > my + 2 ? my + 2 : cj);
+                const size_t o = size_t(ci + 3) * (my + 6) + (cj + 3);
+                if (yin) {
+                    const int d = ii * FS + (jj - H);
+#pragma unroll
+                    for (int m = 0; m < MEQN; m++) S.fs[m * RI * FS + d] = R(0.5 * __ldg(a.Fg + m * a.gplane + o));
+                }
+                if (xin) {
+                    const int d = (ii - H) * RJ + jj;
+#pragma unroll
+                    for (int m = 0; m < MEQN; m++) S.gs[m * TI * RJ + d] = R(0.5 * __ldg(a.Gg + m * a.gplane + o));
+                }
+                return;
             }
-        }
-#pragma unroll
-        for (int it = 0; it < NIT; it++) {
-            const int e = tid + it * NT;
-            const int ii = e / RJ, jj = e - ii * RJ;
-            const bool xin = ii >= H && ii < H + TI, yin = jj >= H && jj < H + TJ;
-            if (e < PQ && (xin || yin)) {
-#pragma unroll
-                for (int m = 0; m < MEQN; m++) qs[m * PQ + e] = R(v[it][m]);
-            }
-        }
-        __syncthreads();
-    }
-
-    // ---- phase 1: per cell of the cross region: FluxFunc (FluxFunc.cpp:19-42,
-    // once per cell instead of once per stencil point of every face), halved
-    // for the LLF split, and the cell's u, v, p, c for SetWaveSpd.cpp:24-50 ----
-    for (int e = tid; e < PQ; e += NT) {
-        const int ii = e / RJ, jj = e - ii * RJ;
-        const bool xin = ii >= H && ii < H + TI, yin = jj >= H && jj < H + TJ;
-        if (!xin && !yin) continue;
-        R rho, m1, m2, m3, en;
-        {
-            rho = qs[e]; m1 = qs[PQ + e]; m2 = qs[2 * PQ + e]; m3 = qs[3 * PQ + e]; en = qs[4 * PQ + e];
-        }
-        const R ir = rcp(rho);
-        const R u1 = m1 * ir, u2 = m2 * ir, u3 = m3 * ir;
-        const R press = (gamma - R(1)) * (en - R(0.5) * rho * (u1 * u1 + u2 * u2 + u3 * u3));
-        {
-            prim[e] = u1;
-            prim[PQ + e] = u2;
-            prim[2 * PQ + e] = press;
-            prim[3 * PQ + e] = fsqrt(fabs(gamma * press * ir));
-        }
-        if (FG) {
-            // 0.5 * F, 0.5 * G of the integrated-flux kernel, unremapped: it
-            // covers the 3-cell ghost frame; cells of a partial tile beyond it
-            // only feed discarded faces, so their index is clamped.
-            int ci = i0 + ii - H, cj = j0 + jj - H;
-            ci = ci < -3 ? -3 : (ci > mx + 2 ? mx + 2 : ci);
-            cj = cj < -3 ? -3 : (cj > my + 2 ? my + 2 : cj);
-            const size_t o = size_t(ci + 3) * (my + 6) + (cj + 3);
+            const R hr = R(0.5) * rho, hep = R(0.5) * (en + press);
             if (yin) {
-                const int d = ii * FS + (jj - H);
-#pragma unroll
-                for (int m = 0; m < MEQN; m++) fs[m * RI * FS + d] = R(0.5 * __ldg(a.Fg + m * a.gplane + o));
+                const int o = ii * FS + (jj - H);
+                S.fs[o] = hr * u1;
+                S.fs[RI * FS + o] = hr * u1 * u1 + R(0.5) * press;
+                S.fs[2 * RI * FS + o] = hr * u1 * u2;
+                S.fs[3 * RI * FS + o] = hr * u1 * u3;
+                S.fs[4 * RI * FS + o] = u1 * hep;
             }
             if (xin) {
-                const int d = (ii - H) * RJ + jj;
-#pragma unroll
-                for (int m = 0; m < MEQN; m++) gs[m * TI * RJ + d] = R(0.5 * __ldg(a.Gg + m * a.gplane + o));
+                const int o = (ii - H) * RJ + jj;
+                S.gs[o] = hr * u2;
+                S.gs[TI * RJ + o] = hr * u2 * u1;
+                S.gs[2 * TI * RJ + o] = hr * u2 * u2 + R(0.5) * press;
+                S.gs[3 * TI * RJ + o] = hr * u2 * u3;
+                S.gs[4 * TI * RJ + o] = u2 * hep;
             }
-            continue;
-        }
-        const R hr = R(0.5) * rho, hep = R(0.5) * (en + press);
-        if (yin) {
-            const int o = ii * FS + (jj - H);
-            fs[o] = hr * u1;
-            fs[RI * FS + o] = hr * u1 * u1 + R(0.5) * press;
-            fs[2 * RI * FS + o] = hr * u1 * u2;
-            fs[3 * RI * FS + o] = hr * u1 * u3;
-            fs[4 * RI * FS + o] = u1 * hep;
-        }
-        if (xin) {
-            const int o = (ii - H) * RJ + jj;
-            gs[o] = hr * u2;
-            gs[TI * RJ + o] = hr * u2 * u1;
-            gs[2 * TI * RJ + o] = hr * u2 * u2 + R(0.5) * press;
-            gs[3 * TI * RJ + o] = hr * u2 * u3;
-            gs[4 * TI * RJ + o] = u2 * hep;
+        };
+        R v[NV][MEQN];
+        if constexpr (NV > 1) {
+#pragma unroll
+            for (int it = 0; it < NIT; it++) load(tid + it * NT, v[it]);
+#pragma unroll
+            for (int it = 0; it < NIT; it++) cell(tid + it * NT, v[it]);
+        } else {
+            for (int e = tid; e < PQ; e += NT) {
+                load(e, v[0]);
+                cell(e, v[0]);
+            }
         }
     }
     __syncthreads();
 
-    // ---- phase 2: one thread per face (x faces then y faces) ----
-#define eps (Par<R>::eps(a))
-#define pw (Par<R>::pw(a))
-    const R ag1 = a.alpha_in ? R(a.alpha_in[0]) : R(0);
-    const R ag2 = a.alpha_in ? R(a.alpha_in[1]) : R(0);
-    R smax_x = R(0), smax_y = R(0);
+    // ---- phase 2: one thread per face, x faces then y faces ----
+    double smax_x = 0.0, smax_y = 0.0;
     bool neg = false, nonfinite = false;
-    const int nwork = Cfg::NFX + Cfg::NFY;
+    {
+        const R ag1 = a.alpha_in ? R(a.alpha_in[0]) : R(0);
 #pragma unroll 1
-    for (int k = tid; k < nwork; k += NT) {
-        const int w = k;
-        const bool isx = w < Cfg::NFX;
-        int fi, fj, qbase, qstr, fbase, fstr, fplane;
-        const R* fl;
-        if (isx) {
-            // face between rows fi-1, fi of the tile
-            if constexpr (Cfg::template XROW8<R>()) {
-                fi = (w >> 5) + ((w >> 1) & 8); fj = w & 15;   // half-warps on rows r and r + 8
-            } else {
-                fi = w / TJ; fj = w - fi * TJ;
-            }
-            qbase = (H + fi) * RJ + (H + fj); qstr = RJ;
-            fl = fs; fbase = (H + fi) * FS + fj; fstr = FS; fplane = RI * FS;
-        } else {
-            // face between cols fj-1, fj; taken by rows of TJ, then the last
-            // column, so a half-warp reads one row of the staged tile (FP32:
-            // half-warps on rows r and r + 8; the last warp takes row 7 and
-            // the last column)
-            const int v = w - Cfg::NFX;
-            if constexpr (Cfg::template XROW8<R>()) {
-                const int wv = v >> 5, ln = v & 31;
-                if (wv < 7) { fi = wv + (ln & 16 ? 8 : 0); fj = ln & 15; }
-                else if (ln < 16) { fi = 7; fj = ln; }
-                else { fi = ln - 16; fj = TJ; }
-            } else {
-                fi = v < TI * TJ ? v / TJ : v - TI * TJ;
-                fj = v < TI * TJ ? v - fi * TJ : TJ;
-            }
-            qbase = (H + fi) * RJ + (H + fj); qstr = 1;
-            fl = gs; fbase = fi * RJ + (H + fj); fstr = 1; fplane = TI * RJ;
+        for (int k = tid; k < Cfg::NFX; k += NT) {
+            bool in_cfl;
+            const R al = stage_face<R, VER, P2, Cfg, FG, true>(a, S, k, i0, j0, ag1, neg, in_cfl);
+            if (!(al <= R(1e30))) nonfinite = true;
+            else if (in_cfl) smax_x = Max(smax_x, double(al));
         }
-        const int cn = isx ? 1 : 2, ct = isx ? 2 : 1;   // normal / tangential momentum
-        const int ql = qbase - qstr;
-        // Face average (ConstructL.cpp:72-77) in the normal frame.
-        R Qa[MEQN];
-        Qa[0] = R(0.5) * (qs[qbase] + qs[ql]);
-        Qa[1] = R(0.5) * (qs[cn * PQ + qbase] + qs[cn * PQ + ql]);
-        Qa[2] = R(0.5) * (qs[ct * PQ + qbase] + qs[ct * PQ + ql]);
-        Qa[3] = R(0.5) * (qs[3 * PQ + qbase] + qs[3 * PQ + ql]);
-        Qa[4] = R(0.5) * (qs[4 * PQ + qbase] + qs[4 * PQ + ql]);
-        const typename Euler::Eig<R> ev = Euler::eig(gamma, Qa);
-        // SetWaveSpd.cpp:39-68 from the two cells' u_n, p, c (nmag = 1) and
-        // the LLF alpha of ConstructL.cpp:172-174.
-        R alpha;
-        {
-            const int un = isx ? 0 : 1;
-            R unl, unr, pl, pr, cl, cr;
-            {
-                unl = prim[un * PQ + ql]; unr = prim[un * PQ + qbase];
-                pl = prim[2 * PQ + ql]; pr = prim[2 * PQ + qbase];
-                cl = prim[3 * PQ + ql]; cr = prim[3 * PQ + qbase];
-            }
-            const R rho = Qa[0];
-            const R ua = R(0.5) * (unl + unr);
-            const R pa = R(0.5) * (pl + pr);
-            const R ca = fsqrt(fabs(gamma * pa * rcp(rho)));
-            if (pa < R(0) || rho < R(0)) neg = true;
-            const R s1 = Min(unl - cl, ua - ca);
-            const R s2 = Max(unr + cr, ua + ca);
-            alpha = Max(isx ? ag1 : ag2, Max(fabs(s1), fabs(s2)));
-        }
-        if (!(alpha <= R(1e30))) nonfinite = true;
-        // gp = 0.5 (L f + l_alpha L q) = L (0.5 f + 0.5 l_alpha q), points
-        // 0..4; gm the same with -l_alpha, points 5..1 (ConstructL.cpp:179-185).
-        const R lah = R(0.5) * Par<R>::ascale(a) * alpha;
-        const typename Euler::Rows<R> rw = Euler::rows(ev);
-        R fh[MEQN] = {R(0), R(0), R(0), R(0), R(0)};
-        if constexpr (sizeof(R) == 4 && (P2 || VER == FIN_WENO_FD)) {
-            // FP32: the split pairs and the paired reconstructions of
-            // weno_char_flux_x2 (f32x2), the same passes over the fields
-            auto pt = [&](int s, float* q, float* f) {
-                const int oq = qbase + (s - 3) * qstr, of = fbase + (s - 3) * fstr;
-                q[0] = qs[oq]; q[1] = qs[cn * PQ + oq]; q[2] = qs[ct * PQ + oq]; q[3] = qs[3 * PQ + oq];
-                q[4] = qs[4 * PQ + oq];
-                f[0] = fl[of]; f[1] = fl[cn * fplane + of]; f[2] = fl[ct * fplane + of]; f[3] = fl[3 * fplane + of];
-                f[4] = fl[4 * fplane + of];
-            };
-            weno_char_flux_x2<VER>(ev, lah, pt, eps, fh);
-        } else if (FIN_F64_MERGE && sizeof(R) == 8) {
-            // fields 0, 4 and 1 in one sweep of the stencil (left014 shares
-            // the acoustic rows' tail), then fields 2 and 3; the right
-            // projections are added in the same order as the three passes below
-            R p0[5], p4[5], m0[5], m4[5], p1[5], m1[5];
-#pragma unroll
-            for (int s = 0; s < 6; s++) {
-                asm volatile("" ::: "memory");
-                const int oq = qbase + (s - 3) * qstr, of = fbase + (s - 3) * fstr;
-                const R q0 = qs[oq], qn = qs[cn * PQ + oq], qt = qs[ct * PQ + oq], qw = qs[3 * PQ + oq], qe = qs[4 * PQ + oq];
-                const R f0 = fl[of], fn = fl[cn * fplane + of], ft = fl[ct * fplane + of], fw = fl[3 * fplane + of],
-                        fe = fl[4 * fplane + of];
-                if (s < 5) {
-                    const R v[MEQN] = {f0 + lah * q0, fn + lah * qn, ft + lah * qt, fw + lah * qw, fe + lah * qe};
-                    Euler::left014(ev, rw, v, p0[s], p1[s], p4[s]);
-                }
-                if (s > 0) {
-                    const R v[MEQN] = {f0 - lah * q0, fn - lah * qn, ft - lah * qt, fw - lah * qw, fe - lah * qe};
-                    Euler::left014(ev, rw, v, m0[5 - s], m1[5 - s], m4[5 - s]);
-                }
-            }
+        const R ag2 = a.alpha_in ? R(a.alpha_in[1]) : R(0);
 #pragma unroll 1
-            for (int k = 0; k < 3; k++) {
-                R up[5], um[5];
-#pragma unroll
-                for (int t = 0; t < 5; t++) {
-                    up[t] = k == 0 ? p0[t] : (k == 1 ? p4[t] : p1[t]);
-                    um[t] = k == 0 ? m0[t] : (k == 1 ? m4[t] : m1[t]);
-                }
-                right_add<R>(ev, k == 0 ? 0 : (k == 1 ? 4 : 1), weno_pair<R, VER, P2>(up, um, eps, pw), fh);
-            }
-            {
-                // fields 2 and 3 (rows v_t - u2 v0 and v_w - u3 v0)
-                R p2[5], p3[5], m2[5], m3[5];
-#pragma unroll
-                for (int s = 0; s < 6; s++) {
-                    asm volatile("" ::: "memory");
-                    const int oq = qbase + (s - 3) * qstr, of = fbase + (s - 3) * fstr;
-                    const R q0 = qs[oq], qt = qs[ct * PQ + oq], qw = qs[3 * PQ + oq];
-                    const R f0 = fl[of], ft = fl[ct * fplane + of], fw = fl[3 * fplane + of];
-                    if (s < 5) {
-                        const R v0 = f0 + lah * q0;
-                        p2[s] = (ft + lah * qt) - ev.u2 * v0;
-                        p3[s] = (fw + lah * qw) - ev.u3 * v0;
-                    }
-                    if (s > 0) {
-                        const R v0 = f0 - lah * q0;
-                        m2[5 - s] = (ft - lah * qt) - ev.u2 * v0;
-                        m3[5 - s] = (fw - lah * qw) - ev.u3 * v0;
-                    }
-                }
-#pragma unroll 1
-                for (int k = 0; k < 2; k++) {
-                    R up[5], um[5];
-#pragma unroll
-                    for (int t = 0; t < 5; t++) {
-                        up[t] = k == 0 ? p2[t] : p3[t];
-                        um[t] = k == 0 ? m2[t] : m3[t];
-                    }
-                    right_add<R>(ev, k == 0 ? 2 : 3, weno_pair<R, VER, P2>(up, um, eps, pw), fh);
-                }
-            }
-        } else {
-        {
-            // pass 1: characteristic fields 0 and 4 (acoustic rows, shared tail)
-            R p0[5], p4[5], m0[5], m4[5];
-#pragma unroll
-            for (int s = 0; s < 6; s++) {
-                // keep the compiler from hoisting every stencil point's loads
-                // ahead of the arithmetic (that would hold ~60 values live)
-                asm volatile("" ::: "memory");
-                const int oq = qbase + (s - 3) * qstr, of = fbase + (s - 3) * fstr;
-                const R q0 = qs[oq], qn = qs[cn * PQ + oq], qt = qs[ct * PQ + oq], qw = qs[3 * PQ + oq], qe = qs[4 * PQ + oq];
-                const R f0 = fl[of], fn = fl[cn * fplane + of], ft = fl[ct * fplane + of], fw = fl[3 * fplane + of],
-                        fe = fl[4 * fplane + of];
-                if (s < 5) {
-                    const R v[MEQN] = {f0 + lah * q0, fn + lah * qn, ft + lah * qt, fw + lah * qw, fe + lah * qe};
-                    Euler::left04(ev, rw, v, p0[s], p4[s]);
-                }
-                if (s > 0) {
-                    const R v[MEQN] = {f0 - lah * q0, fn - lah * qn, ft - lah * qt, fw - lah * qw, fe - lah * qe};
-                    Euler::left04(ev, rw, v, m0[5 - s], m4[5 - s]);
-                }
-            }
-            // one reconstruction pair per iteration; the loop is not unrolled,
-            // which keeps the scheduler from overlapping the two pairs
-#pragma unroll 1
-            for (int k = 0; k < 2; k++) {
-                R up[5], um[5];
-#pragma unroll
-                for (int t = 0; t < 5; t++) {
-                    up[t] = k == 0 ? p0[t] : p4[t];
-                    um[t] = k == 0 ? m0[t] : m4[t];
-                }
-                right_add<R>(ev, k == 0 ? 0 : 4, weno_pair<R, VER, P2>(up, um, eps, pw), fh);
-            }
-        }
-        {
-            // pass 2: characteristic field 1 (the entropy-like row)
-            R p1[5], m1[5];
-#pragma unroll
-            for (int s = 0; s < 6; s++) {
-                // keep the compiler from hoisting every stencil point's loads
-                // ahead of the arithmetic (that would hold ~60 values live)
-                asm volatile("" ::: "memory");
-                const int oq = qbase + (s - 3) * qstr, of = fbase + (s - 3) * fstr;
-                const R q0 = qs[oq], qn = qs[cn * PQ + oq], qt = qs[ct * PQ + oq], qw = qs[3 * PQ + oq], qe = qs[4 * PQ + oq];
-                const R f0 = fl[of], fn = fl[cn * fplane + of], ft = fl[ct * fplane + of], fw = fl[3 * fplane + of],
-                        fe = fl[4 * fplane + of];
-                if (s < 5) {
-                    const R v[MEQN] = {f0 + lah * q0, fn + lah * qn, ft + lah * qt, fw + lah * qw, fe + lah * qe};
-                    p1[s] = Euler::left1(ev, rw, v);
-                }
-                if (s > 0) {
-                    const R v[MEQN] = {f0 - lah * q0, fn - lah * qn, ft - lah * qt, fw - lah * qw, fe - lah * qe};
-                    m1[5 - s] = Euler::left1(ev, rw, v);
-                }
-            }
-            right_add<R>(ev, 1, weno_pair<R, VER, P2>(p1, m1, eps, pw), fh);
-        }
-        {
-            // pass 3: fields 2 and 3 (rows v_t - u2 v0 and v_w - u3 v0)
-            R p2[5], p3[5], m2[5], m3[5];
-#pragma unroll
-            for (int s = 0; s < 6; s++) {
-                // keep the compiler from hoisting every stencil point's loads
-                // ahead of the arithmetic (that would hold ~60 values live)
-                asm volatile("" ::: "memory");
-                const int oq = qbase + (s - 3) * qstr, of = fbase + (s - 3) * fstr;
-                const R q0 = qs[oq], qt = qs[ct * PQ + oq], qw = qs[3 * PQ + oq];
-                const R f0 = fl[of], ft = fl[ct * fplane + of], fw = fl[3 * fplane + of];
-                if (s < 5) {
-                    const R v0 = f0 + lah * q0;
-                    p2[s] = (ft + lah * qt) - ev.u2 * v0;
-                    p3[s] = (fw + lah * qw) - ev.u3 * v0;
-                }
-                if (s > 0) {
-                    const R v0 = f0 - lah * q0;
-                    m2[5 - s] = (ft - lah * qt) - ev.u2 * v0;
-                    m3[5 - s] = (fw - lah * qw) - ev.u3 * v0;
-                }
-            }
-#pragma unroll 1
-            for (int k = 0; k < 2; k++) {
-                R up[5], um[5];
-#pragma unroll
-                for (int t = 0; t < 5; t++) {
-                    up[t] = k == 0 ? p2[t] : p3[t];
-                    um[t] = k == 0 ? m2[t] : m3[t];
-                }
-                right_add<R>(ev, k == 0 ? 2 : 3, weno_pair<R, VER, P2>(up, um, eps, pw), fh);
-            }
-        }
-        }
-        // Back to (rho, rho u, rho v, rho w, E) and store.
-        if (isx) {
-            const R o[MEQN] = {fh[0], fh[1], fh[2], fh[3], fh[4]};
-#pragma unroll
-            for (int m = 0; m < MEQN; m++) Fh[m * (TI + 1) * TJ + fi * TJ + fj] = o[m];
-            const int gfi = i0 + fi, gj = j0 + fj;
-            if (FG && a.flux_x && gfi <= mx && gj < my) {
-#pragma unroll
-                for (int m = 0; m < MEQN; m++) a.flux_x[(size_t(m) * (mx + 1) + gfi) * my + gj] = double(o[m]);
-            }
-            // GetCFL's Max skips NaN entries (Max(NaN, c) = c), so only
-            // finite face speeds enter the CFL maximum.
-            if (gfi < mx && gj < my && alpha <= R(1e30) && !(FG && a.flux_only && gfi == 0 && gj == 0))
-                smax_x = Max(smax_x, alpha);
-            if (a.face_alpha_x && gfi <= mx && gj < my) a.face_alpha_x[size_t(gfi) * my + gj] = double(alpha);
-        } else {
-            const R o[MEQN] = {fh[0], fh[2], fh[1], fh[3], fh[4]};
-#pragma unroll
-            for (int m = 0; m < MEQN; m++) Gh[m * TI * (TJ + 1) + fi * (TJ + 1) + fj] = o[m];
-            const int gi = i0 + fi, gfj = j0 + fj;
-            if (FG && a.flux_y && gi < mx && gfj <= my) {
-#pragma unroll
-                for (int m = 0; m < MEQN; m++) a.flux_y[(size_t(m) * mx + gi) * (my + 1) + gfj] = double(o[m]);
-            }
-            if (gi < mx && gfj < my && alpha <= R(1e30) && !(FG && a.flux_only && gi == 0 && gfj == 0))
-                smax_y = Max(smax_y, alpha);
-            if (a.face_alpha_y && gi < mx && gfj <= my) a.face_alpha_y[size_t(gi) * (my + 1) + gfj] = double(alpha);
+        for (int k = tid; k < Cfg::NFY; k += NT) {
+            bool in_cfl;
+            const R al = stage_face<R, VER, P2, Cfg, FG, false>(a, S, k, i0, j0, ag2, neg, in_cfl);
+            if (!(al <= R(1e30))) nonfinite = true;
+            else if (in_cfl) smax_y = Max(smax_y, double(al));
         }
     }
+    if (OPND) asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-#undef gamma
-#undef eps
-#undef pw
 
     // ---- phase 3: flux difference, stage update, next-stage wave speed ----
     double cs_x = 0.0, cs_y = 0.0;
@@ -703,10 +670,21 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const int i0, con
         // B as far as the compiler knows, so loads interleaved with the
         // stores would wait one memory round trip per component
         double va[MEQN], vb[MEQN];
+        if constexpr (OPND) {
+            const R* const qc = S.qs + (H + ci) * RJ + (H + cj);
 #pragma unroll
-        for (int m = 0; m < MEQN; m++) {
-            va[m] = a.A ? a.A[m * a.plane + g] : 0.0;
-            vb[m] = a.B ? a.B[m * a.plane + g] : 0.0;
+            for (int m = 0; m < MEQN; m++) {
+                const double own = qc[m * PQ], oth = ext ? S.opnd[m * TI * TJ + c] : 0.0;
+                va[m] = a.A == a.qin ? own : oth;
+                // A and B apart from each other and from q_in: B is not staged
+                vb[m] = a.B == a.qin ? own : (a.B == ext ? oth : (a.B ? a.B[m * a.plane + g] : 0.0));
+            }
+        } else {
+#pragma unroll
+            for (int m = 0; m < MEQN; m++) {
+                va[m] = a.A ? a.A[m * a.plane + g] : 0.0;
+                vb[m] = a.B ? a.B[m * a.plane + g] : 0.0;
+            }
         }
         double qn[MEQN];
 #pragma unroll
@@ -714,8 +692,8 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const int i0, con
             // ConstructL.cpp:396-398
             // (the FP32 forms difference their FP32 fluxes in FP32 and widen
             // the result once)
-            const R f1 = Fh[m * (TI + 1) * TJ + (ci + 1) * TJ + cj], f0 = Fh[m * (TI + 1) * TJ + ci * TJ + cj];
-            const R g1 = Gh[m * TI * (TJ + 1) + ci * (TJ + 1) + cj + 1], g0 = Gh[m * TI * (TJ + 1) + ci * (TJ + 1) + cj];
+            const R f1 = S.Fh[m * (TI + 1) * TJ + (ci + 1) * TJ + cj], f0 = S.Fh[m * (TI + 1) * TJ + ci * TJ + cj];
+            const R g1 = S.Gh[m * TI * (TJ + 1) + ci * (TJ + 1) + cj + 1], g0 = S.Gh[m * TI * (TJ + 1) + ci * (TJ + 1) + cj];
             R Lr = -(f1 - f0) * R(a.rdx);
             Lr = Lr - (g1 - g0) * R(a.rdy);
             const double L = double(Lr);
@@ -729,13 +707,14 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const int i0, con
             a.qout[m * a.plane + g] = v;
         }
         if (a.alpha_out) {
-            // GlobalWaveSpd.cpp:71-76 on the new state, both directions.
-            // The FP32 forms use it only as the FP32 LLF speed of the next
-            // stage, so they evaluate it in FP32.
+            // GlobalWaveSpd.cpp:71-76 on the new state, both directions:
+            // max(|u_n - c|, |u_n + c|) = |u_n| + c.  The FP32 forms use it
+            // only as the FP32 LLF speed of the next stage, so they evaluate
+            // it in FP32.
             const R qx[MEQN] = {R(qn[0]), R(qn[1]), R(qn[2]), R(qn[3]), R(qn[4])};
-            const R qy[MEQN] = {qx[0], qx[2], qx[1], qx[3], qx[4]};
-            const double sx = double(Euler::cell_speed(Euler::cell(R(gam), qx)));
-            const double sy = double(Euler::cell_speed(Euler::cell(R(gam), qy)));
+            const typename Euler::Cell<R> w = Euler::cell(R(gam), qx);
+            const double sx = double(fabs(w.un) + w.c);
+            const double sy = double(fabs(qx[2] * rcp(qx[0])) + w.c);
             if (!(sx <= 1e300) || !(sy <= 1e300)) nonfinite = true;
             if (sx <= 1e300) cs_x = Max(cs_x, sx);
             if (sy <= 1e300) cs_y = Max(cs_y, sy);
@@ -743,26 +722,20 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const int i0, con
     }
 
     // ---- block reductions of the four maxima, one atomic each ----
-    double v4[4] = {double(smax_x), double(smax_y), cs_x, cs_y};
+    // Non-finite speeds were flagged per value above (a NaN does not survive
+    // Max(NaN, b) = b), so the reduction only sees finite ones.
+    const double v4[4] = {smax_x, smax_y, cs_x, cs_y};
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-        // Non-finite speeds were flagged per value above (a NaN does not
-        // survive Max(NaN, b) = b), so the reduction only sees finite ones.
-        double v = v4[k] <= 1e300 ? v4[k] : 0.0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v = Max(v, __shfl_xor_sync(0xffffffffu, v, o));
-        v4[k] = v;
-    }
-    if ((tid & 31) == 0) {
-#pragma unroll
-        for (int k = 0; k < 4; k++) red[(tid >> 5) * 4 + k] = v4[k];
+        const double v = warp_max_nonneg(v4[k] <= 1e300 ? v4[k] : 0.0);
+        if ((tid & 31) == 0) S.red[(tid >> 5) * 4 + k] = v;
     }
     if (neg) atomicOr(a.status, 2u);
     if (nonfinite) atomicOr(a.status, 1u);
     __syncthreads();
     if (tid < 4) {
         double v = 0.0;
-        for (int wv = 0; wv < NT / 32; wv++) v = Max(v, red[wv * 4 + tid]);
+        for (int wv = 0; wv < NT / 32; wv++) v = Max(v, S.red[wv * 4 + tid]);
         double* dst = tid < 2 ? a.smax_out : a.alpha_out;
         if (dst) atomic_max_nonneg(dst + (tid & 1), v);
     }

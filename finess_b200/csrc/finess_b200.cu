@@ -46,8 +46,8 @@ int set_err(int code, const std::string& msg)
             return set_err(FIN_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
     } while (0)
 
-// Tile shape of the stage kernel: 16 x 16 cells, 544 faces over 288 threads
-// (two rounds of the face loop, the second 89% full).
+// Tile shape of the stage kernels: 15 x 16 cells, so the 256 x faces and the
+// 255 y faces take one round of the 256 threads each.
 #ifndef FIN_TILE_TI
 #define FIN_TILE_TI 15
 #define FIN_TILE_TJ 16
