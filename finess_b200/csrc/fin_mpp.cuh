@@ -5,7 +5,10 @@
 // (apps/2d/euler/lib/ApplyMPPLimiter2D.cpp:27-285) and the conservative
 // update of FinSolveLxW.cpp:143-151.
 //
-// Two kernels, one thread per cell:
+// Two kernels, one thread per cell of a 16 x 16 tile whose states and fluxes
+// sit in shared memory (each cell's three divisions once, not once per face
+// and component: the update kernel 0.130 -> 0.071 ms at 1023 x 1025; both are
+// now bound by the latency of their flux loads):
 //   k_mpp_limit   the cell's four limiting factors amin[k] (k = left, right,
 //                 bottom, top face): the density step (:57-92) and the
 //                 pressure step over the 16 on/off combinations of the faces
@@ -15,7 +18,7 @@
 //                 theta (fhat - fLF) + fLF (:248-270), the update, and the
 //                 new state's global wave speeds (GlobalWaveSpd.cpp:71-76).
 // The Lax-Friedrichs fluxes are recomputed where needed (cheap) instead of
-// stored.  Every operation follows the reference's order with correctly
+// stored.  Every operation that enters a result follows the reference's order with correctly
 // rounded IEEE operations (no contraction), so equal inputs give equal
 // results.
 #pragma once
@@ -46,66 +49,77 @@ struct MppArgs {
     unsigned int* status; // bit 0: non-finite wave speed of q^{n+1}
 };
 
-// FluxFunc.cpp:19-42, component m of direction d (0: f, 1: g).
-__device__ __forceinline__ double flux_comp(const double* Q, double gamma, int d, int m)
+// A block's TI x TJ cells with one cell around them: states and fluxes
+// (FluxFunc.cpp:19-42) of the cross region, each evaluated once.  The f and g
+// arrays hold the rows (columns) that the tile's x (y) faces read.
+constexpr int TI = 16, TJ = 16, NT = TI * TJ, CI = TI + 2, CJ = TJ + 2;
+struct Tile {
+    double q[MEQN][CI][CJ];
+    double f[MEQN][CI][TJ];
+    double g[MEQN][TI][CJ];
+};
+
+__device__ __forceinline__ void load_tile(const MppArgs& a, Tile& T, int i0, int j0)
 {
-    const double rho = Q[0];
-    const double u1 = dvd(Q[1], rho), u2 = dvd(Q[2], rho), u3 = dvd(Q[3], rho);
-    const double energy = Q[4];
-    const double ke = add(add(mul(u1, u1), mul(u2, u2)), mul(u3, u3));
-    const double press = mul(sub(gamma, 1.0e0), sub(energy, mul(mul(0.5e0, rho), ke)));
-    const double un = d == 0 ? u1 : u2;
-    switch (m) {
-    case 0: return mul(rho, un);
-    case 1: return d == 0 ? add(mul(mul(rho, u1), u1), press) : mul(mul(rho, u2), u1);
-    case 2: return d == 0 ? mul(mul(rho, u1), u2) : add(mul(mul(rho, u2), u2), press);
-    case 3: return mul(mul(rho, un), u3);
-    default: return mul(un, add(energy, press));
+    for (int e = threadIdx.x; e < CI * CJ; e += NT) {
+        const int ii = e / CJ, jj = e - ii * CJ;
+        const bool xin = ii >= 1 && ii <= TI, yin = jj >= 1 && jj <= TJ;
+        if (!xin && !yin) continue;
+        const size_t o = size_t(bc_remap(i0 + ii - 1, a.mx, a.bc[0], a.bc[1])) * a.my +
+                         bc_remap(j0 + jj - 1, a.my, a.bc[2], a.bc[3]);
+        double Q[MEQN];
+#pragma unroll
+        for (int m = 0; m < MEQN; m++) {
+            Q[m] = a.q[m * a.plane + o];
+            T.q[m][ii][jj] = Q[m];
+        }
+        const double rho = Q[0];
+        const double u1 = dvd(Q[1], rho), u2 = dvd(Q[2], rho), u3 = dvd(Q[3], rho);
+        const double energy = Q[4];
+        const double ke = add(add(mul(u1, u1), mul(u2, u2)), mul(u3, u3));
+        const double press = mul(sub(a.gamma, 1.0e0), sub(energy, mul(mul(0.5e0, rho), ke)));
+        if (yin) {
+            const int c = jj - 1;
+            T.f[0][ii][c] = mul(rho, u1);
+            T.f[1][ii][c] = add(mul(mul(rho, u1), u1), press);
+            T.f[2][ii][c] = mul(mul(rho, u1), u2);
+            T.f[3][ii][c] = mul(mul(rho, u1), u3);
+            T.f[4][ii][c] = mul(u1, add(energy, press));
+        }
+        if (xin) {
+            const int r = ii - 1;
+            T.g[0][r][jj] = mul(rho, u2);
+            T.g[1][r][jj] = mul(mul(rho, u2), u1);
+            T.g[2][r][jj] = add(mul(mul(rho, u2), u2), press);
+            T.g[3][r][jj] = mul(mul(rho, u2), u3);
+            T.g[4][r][jj] = mul(u2, add(energy, press));
+        }
     }
 }
 
-__device__ __forceinline__ void load_cell(const MppArgs& a, int i, int j, double* Q)
+// Lax-Friedrichs flux of the face between cells L and R, one component
+// (ConstructLFL.cpp:92-108): 0.5 (f(L) + f(R)) + 0.5 alpha (q_L - q_R).
+__device__ __forceinline__ double lf(double fL, double fR, double qL, double qR, double alpha)
 {
-    const size_t g = size_t(bc_remap(i, a.mx, a.bc[0], a.bc[1])) * a.my + bc_remap(j, a.my, a.bc[2], a.bc[3]);
-#pragma unroll
-    for (int m = 0; m < MEQN; m++) Q[m] = a.q[m * a.plane + g];
+    return add(mul(0.5, add(fL, fR)), mul(mul(0.5, alpha), sub(qL, qR)));
 }
 
-// Lax-Friedrichs flux of the face between cells L and R (ConstructLFL.cpp:
-// 92-108): 0.5 (f(L) + f(R)) + 0.5 alpha (q_L - q_R), all components.
-__device__ __forceinline__ void lf_flux(const double* QL, const double* QR, double gamma, int d, double alpha,
-                                        double* out)
+// The four faces of tile cell (ci, cj), component m: high-order and
+// Lax-Friedrichs fluxes (k = 0: x face i, 1: x face i+1, 2: y face j, 3: y
+// face j+1).
+__device__ __forceinline__ void cell_faces(const MppArgs& a, const Tile& T, int i, int j, int ci, int cj, int m,
+                                           double ax, double ay, double (&fh)[4], double (&fl)[4])
 {
-#pragma unroll
-    for (int m = 0; m < MEQN; m++) {
-        const double fl = flux_comp(QL, gamma, d, m), fr = flux_comp(QR, gamma, d, m);
-        out[m] = add(mul(0.5, add(fl, fr)), mul(mul(0.5, alpha), sub(QL[m], QR[m])));
-    }
-}
-
-// The four faces of cell (i, j): high-order and Lax-Friedrichs fluxes
-// (k = 0: x face i, 1: x face i+1, 2: y face j, 3: y face j+1).
-__device__ __forceinline__ void cell_faces(const MppArgs& a, int i, int j, double (&fh)[4][MEQN],
-                                           double (&fl)[4][MEQN], double (&qc)[MEQN])
-{
+    const double qc = T.q[m][ci + 1][cj + 1];
+    fl[0] = lf(T.f[m][ci][cj], T.f[m][ci + 1][cj], T.q[m][ci][cj + 1], qc, ax);
+    fl[1] = lf(T.f[m][ci + 1][cj], T.f[m][ci + 2][cj], qc, T.q[m][ci + 2][cj + 1], ax);
+    fl[2] = lf(T.g[m][ci][cj], T.g[m][ci][cj + 1], T.q[m][ci + 1][cj], qc, ay);
+    fl[3] = lf(T.g[m][ci][cj + 1], T.g[m][ci][cj + 2], qc, T.q[m][ci + 1][cj + 2], ay);
     const int mx = a.mx, my = a.my;
-    double Qn[MEQN];
-    load_cell(a, i, j, qc);
-    load_cell(a, i - 1, j, Qn);
-    lf_flux(Qn, qc, a.gamma, 0, a.alpha[0], fl[0]);
-    load_cell(a, i + 1, j, Qn);
-    lf_flux(qc, Qn, a.gamma, 0, a.alpha[0], fl[1]);
-    load_cell(a, i, j - 1, Qn);
-    lf_flux(Qn, qc, a.gamma, 1, a.alpha[1], fl[2]);
-    load_cell(a, i, j + 1, Qn);
-    lf_flux(qc, Qn, a.gamma, 1, a.alpha[1], fl[3]);
-#pragma unroll
-    for (int m = 0; m < MEQN; m++) {
-        fh[0][m] = a.fhat[(size_t(m) * (mx + 1) + i) * my + j];
-        fh[1][m] = a.fhat[(size_t(m) * (mx + 1) + i + 1) * my + j];
-        fh[2][m] = a.ghat[(size_t(m) * mx + i) * (my + 1) + j];
-        fh[3][m] = a.ghat[(size_t(m) * mx + i) * (my + 1) + j + 1];
-    }
+    fh[0] = a.fhat[(size_t(m) * (mx + 1) + i) * my + j];
+    fh[1] = a.fhat[(size_t(m) * (mx + 1) + i + 1) * my + j];
+    fh[2] = a.ghat[(size_t(m) * mx + i) * (my + 1) + j];
+    fh[3] = a.ghat[(size_t(m) * mx + i) * (my + 1) + j + 1];
 }
 
 // Pressure of a state, ApplyMPPLimiter2D.cpp:108-113.
@@ -117,40 +131,29 @@ __device__ __forceinline__ double pressure(const double* Q, double gm1)
     return mul(gm1, sub(Q[4], mul(mul(0.5, rho), ke)));
 }
 
-__global__ void __launch_bounds__(128) k_mpp_limit(const MppArgs a)
+// The pressure step's rescaling factors, ApplyMPPLimiter2D.cpp:97-217: for
+// each of the 16 on/off combinations of the faces the state with those faces'
+// (density-limited) high-order fluxes, bisected against the Lax-Friedrichs
+// state when its pressure is negative.  Run by the cells whose states
+// k_mpp_limit could not show to be positive.
+__device__ __noinline__ void pressure_step(const MppArgs& a, const Tile& T, int i, int j, int ci, int cj, double dtx,
+                                           double dty, const double* amin, double* rescale2)
 {
-    const int mx = a.mx, my = a.my;
-    const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (c >= (long long)mx * my) return;
-    const int i = int(c / my), j = int(c - (long long)i * my);
-    double fh[4][MEQN], fl[4][MEQN], qc[MEQN];
-    cell_faces(a, i, j, fh, fl, qc);
-    const double eps = 1.0e-12, rho_min = eps;
-    const double dtx = dvd(a.dt, a.dx), dty = dvd(a.dt, a.dy);
-    const double gm1 = sub(a.gamma, 1.0);
-    // ---- step 1: density (:57-92) ----
-    const double gmin = sub(rho_min, add(add(qc[0], mul(dtx, sub(fl[0][0], fl[1][0]))),
-                                         mul(dty, sub(fl[2][0], fl[3][0]))));
-    double ff[4], amin[4];
-    ff[0] = mul(dtx, sub(fh[0][0], fl[0][0]));
-    ff[1] = mul(-dtx, sub(fh[1][0], fl[1][0]));
-    ff[2] = mul(dty, sub(fh[2][0], fl[2][0]));
-    ff[3] = mul(-dty, sub(fh[3][0], fl[3][0]));
-    int isgn[4];
+    const double ax = a.alpha[0], ay = a.alpha[1], gm1 = sub(a.gamma, 1.0);
+    double fh[4 * MEQN], fl[4 * MEQN], qc[MEQN], qlf[MEQN];
 #pragma unroll
-    for (int k = 0; k < 4; k++) isgn[k] = ff[k] < 0.0 ? 1 : 0;
-    double ffsum = mul(double(isgn[0]), ff[0]);
+    for (int m = 0; m < MEQN; m++) {
+        double h[4], l[4];
+        cell_faces(a, T, i, j, ci, cj, m, ax, ay, h, l);
 #pragma unroll
-    for (int k = 1; k < 4; k++) ffsum = add(ffsum, mul(double(isgn[k]), ff[k]));
-#pragma unroll
-    for (int k = 0; k < 4; k++) amin[k] = isgn[k] == 1 ? Mn(dvd(gmin, sub(ffsum, eps)), 1.e0) : 1.e0;
-    // ---- step 2: pressure (:97-217) ----
-    double qlf[MEQN];
-#pragma unroll
-    for (int m = 0; m < MEQN; m++)
-        qlf[m] = add(add(qc[m], mul(dtx, sub(fl[0][m], fl[1][m]))), mul(dty, sub(fl[2][m], fl[3][m])));
+        for (int k = 0; k < 4; k++) {
+            fh[k * MEQN + m] = h[k];
+            fl[k * MEQN + m] = l[k];
+        }
+        qc[m] = T.q[m][ci + 1][cj + 1];
+        qlf[m] = add(add(qc[m], mul(dtx, sub(l[0], l[1]))), mul(dty, sub(l[2], l[3])));
+    }
     if (pressure(qlf, gm1) < 0.0) atomicOr(a.status, 2u);   // "Negative solution in Lax-Friedrich's flux"
-    double rescale[16];
 #pragma unroll 1
     for (int combo = 0; combo < 16; combo++) {
         // combo bits (i1 i2 i3 i4) with i1 the most significant, as the
@@ -163,16 +166,15 @@ __global__ void __launch_bounds__(128) k_mpp_limit(const MppArgs a)
         for (int m = 0; m < MEQN; m++) {
             double f4[4];
 #pragma unroll
-            for (int k = 0; k < 4; k++) f4[k] = add(mul(aa[k], fh[k][m]), mul(sub(1.0, aa[k]), fl[k][m]));
+            for (int k = 0; k < 4; k++) f4[k] = add(mul(aa[k], fh[k * MEQN + m]), mul(sub(1.0, aa[k]), fl[k * MEQN + m]));
             qh[m] = add(add(qc[m], mul(dtx, sub(f4[0], f4[1]))), mul(dty, sub(f4[2], f4[3])));
         }
         double phigh = pressure(qh, gm1);
-        double r = 1.0;
         if (phigh < 0.0) {
             double root1 = 0.0, root2 = 1.0, rate = 0.0;
 #pragma unroll 1
             for (int nn = 1; nn < 10; nn++) {
-                rate = dvd(add(root1, root2), 2.0);
+                rate = mul(add(root1, root2), 0.5);
                 double q2[MEQN];
 #pragma unroll
                 for (int m = 0; m < MEQN; m++) q2[m] = add(mul(rate, qh[m]), mul(sub(1.0, rate), qlf[m]));
@@ -180,36 +182,113 @@ __global__ void __launch_bounds__(128) k_mpp_limit(const MppArgs a)
                 if (phigh < 0.0) root2 = rate;
                 else root1 = rate;
             }
-            r = phigh > 0.0 ? rate : root1;
+            const double r = phigh > 0.0 ? rate : root1;
+            // :220-227: each face's factor is the least over the combinations it is on in
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (on[k]) rescale2[k] = Mn(rescale2[k], r);
         }
-        rescale[combo] = r;
     }
-    double rescale2[4] = {1.0, 1.0, 1.0, 1.0};
+}
+
+// The cell's four factors.  Bound by memory (fluxes and states once); the
+// pressure step's 16 candidate states a cell, each with three correctly
+// rounded divisions, took 0.33 ms at 1023 x 1025 when every cell ran them,
+// against 0.078 ms with the test below that all sixteen are positive.
+//
+// Every candidate is q_LF plus a subset of the faces' contributions d_k =
+// +-amin_k dt/dx (fhat_k - fLF_k), so its components lie within mid +- rad,
+// mid = q_LF + sum d_k / 2, rad = sum |d_k| / 2.  With rad widened by 1e-13 of
+// the sum of the magnitudes that enter (a thousand roundings), rho_min > 0
+// and 2 rho_min E_min > (1 + 1e-11) max |m|^2 mean that the pressure the
+// reference's formula computes for each candidate is not negative, so every
+// rescaling factor is 1 and no candidate need be formed: the same factors bit
+// for bit.  Cells that fail the test (near-vacuum ones) take pressure_step.
+__global__ void __launch_bounds__(NT, 4) k_mpp_limit(const MppArgs a)
+{
+    __shared__ Tile T;
+    const int mx = a.mx, my = a.my;
+    const int i0 = int(blockIdx.y) * TI, j0 = int(blockIdx.x) * TJ;
+    load_tile(a, T, i0, j0);
+    __syncthreads();
+    const int ci = threadIdx.x / TJ, cj = threadIdx.x - ci * TJ;
+    const int i = i0 + ci, j = j0 + cj;
+    if (i >= mx || j >= my) return;
+    const double ax = a.alpha[0], ay = a.alpha[1];
+    const double eps = 1.0e-12, rho_min = eps;
+    const double dtx = dvd(a.dt, a.dx), dty = dvd(a.dt, a.dy);
+    // component m's bounds over the candidates, from its faces' fluxes
+    double amin[4];
+    auto bounds = [&](int m, const double (&fh)[4], const double (&fl)[4], double& mid, double& rad) {
+        const double qc = T.q[m][ci + 1][cj + 1];
+        const double d0 = amin[0] * dtx * (fh[0] - fl[0]), d1 = amin[1] * dtx * (fl[1] - fh[1]);
+        const double d2 = amin[2] * dty * (fh[2] - fl[2]), d3 = amin[3] * dty * (fl[3] - fh[3]);
+        mid = qc + dtx * (fl[0] - fl[1]) + dty * (fl[2] - fl[3]) + 0.5 * ((d0 + d1) + (d2 + d3));
+        const double mag = fabs(qc) + dtx * ((fabs(fl[0]) + fabs(fl[1])) + (fabs(fh[0]) + fabs(fh[1]))) +
+                           dty * ((fabs(fl[2]) + fabs(fl[3])) + (fabs(fh[2]) + fabs(fh[3])));
+        rad = 0.5 * ((fabs(d0) + fabs(d1)) + (fabs(d2) + fabs(d3))) + 1e-13 * mag;
+    };
+    double rmin, ratio;
+    {
+        double fh[4], fl[4];
+        cell_faces(a, T, i, j, ci, cj, 0, ax, ay, fh, fl);
+        // ---- step 1: density (:57-92) ----
+        const double gmin = sub(rho_min, add(add(T.q[0][ci + 1][cj + 1], mul(dtx, sub(fl[0], fl[1]))),
+                                             mul(dty, sub(fl[2], fl[3]))));
+        double ff[4];
+        ff[0] = mul(dtx, sub(fh[0], fl[0]));
+        ff[1] = mul(-dtx, sub(fh[1], fl[1]));
+        ff[2] = mul(dty, sub(fh[2], fl[2]));
+        ff[3] = mul(-dty, sub(fh[3], fl[3]));
+        int isgn[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) isgn[k] = ff[k] < 0.0 ? 1 : 0;
+        double ffsum = mul(double(isgn[0]), ff[0]);
+#pragma unroll
+        for (int k = 1; k < 4; k++) ffsum = add(ffsum, mul(double(isgn[k]), ff[k]));
+        // gmin / (ffsum - eps) with a negative denominator: at least 1, and so
+        // cut to 1, exactly when gmin does not exceed it
+        const double den = sub(ffsum, eps);
+        ratio = gmin <= den && den < 0.0 ? 1.0 : Mn(dvd(gmin, den), 1.e0);
+#pragma unroll
+        for (int k = 0; k < 4; k++) amin[k] = isgn[k] == 1 ? ratio : 1.e0;
+        double mid, rad;
+        bounds(0, fh, fl, mid, rad);
+        rmin = mid - rad;
+    }
+    // ---- step 2: pressure (:97-217) ----
+    double m2 = 0.0, emin = 0.0;
 #pragma unroll 1
-    for (int t = 0; t < 8; t++) {   // (i1, i2, i3) of :220-227, i3 fastest
-        const int b1 = (t >> 2) & 1, b2 = (t >> 1) & 1, b3 = t & 1;
-        rescale2[0] = Mn(rescale2[0], rescale[8 | (b1 << 2) | (b2 << 1) | b3]);
-        rescale2[1] = Mn(rescale2[1], rescale[(b1 << 3) | 4 | (b2 << 1) | b3]);
-        rescale2[2] = Mn(rescale2[2], rescale[(b1 << 3) | (b2 << 2) | 2 | b3]);
-        rescale2[3] = Mn(rescale2[3], rescale[(b1 << 3) | (b2 << 2) | (b3 << 1) | 1]);
+    for (int m = 1; m < MEQN; m++) {
+        double fh[4], fl[4], mid, rad;
+        cell_faces(a, T, i, j, ci, cj, m, ax, ay, fh, fl);
+        bounds(m, fh, fl, mid, rad);
+        const double w = fabs(mid) + rad;
+        if (m < 4) m2 += w * w;
+        else emin = mid - rad;
     }
-    const size_t nc = size_t(mx) * my;
+    const bool positive = rmin > 0.0 && 2.0 * rmin * emin > (1.0 + 1e-11) * m2 && ratio >= 0.0;
+    double rescale2[4] = {1.0, 1.0, 1.0, 1.0};
+    if (!positive) pressure_step(a, T, i, j, ci, cj, dtx, dty, amin, rescale2);
+    const size_t nc = size_t(mx) * my, c = size_t(i) * my + j;
 #pragma unroll
     for (int k = 0; k < 4; k++) a.amin[k * nc + c] = mul(rescale2[k], amin[k]);
 }
 
-__global__ void __launch_bounds__(128) k_mpp_update(const MppArgs a)
+__global__ void __launch_bounds__(NT) k_mpp_update(const MppArgs a)
 {
-    __shared__ double red[2][4];
+    __shared__ Tile T;
+    __shared__ double red[2][NT / 32];
     const int mx = a.mx, my = a.my;
-    const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const int i0 = int(blockIdx.y) * TI, j0 = int(blockIdx.x) * TJ;
+    load_tile(a, T, i0, j0);
+    __syncthreads();
+    const int ci = threadIdx.x / TJ, cj = threadIdx.x - ci * TJ;
+    const int i = i0 + ci, j = j0 + cj;
     double sx = 0.0, sy = 0.0;
     bool nonfinite = false;
-    if (c < (long long)mx * my) {
-        const int i = int(c / my), j = int(c - (long long)i * my);
-        const size_t nc = size_t(mx) * my;
-        double fh[4][MEQN], fl[4][MEQN], qc[MEQN];
-        cell_faces(a, i, j, fh, fl, qc);
+    if (i < mx && j < my) {
+        const size_t nc = size_t(mx) * my, c = size_t(i) * my + j;
         // face factors (:222-243): min of the two cells' entries, the
         // cell's own at the domain boundary
         const double* am = a.amin;
@@ -219,17 +298,19 @@ __global__ void __launch_bounds__(128) k_mpp_update(const MppArgs a)
         th[2] = j > 0 ? Mn(am[2 * nc + c], am[3 * nc + (c - 1)]) : am[2 * nc + c];
         th[3] = j < my - 1 ? Mn(am[2 * nc + (c + 1)], am[3 * nc + c]) : am[3 * nc + c];
         const double dtdx = dvd(a.dt, a.dx), dtdy = dvd(a.dt, a.dy);
+        const double ax = a.alpha[0], ay = a.alpha[1];
         double qn[MEQN];
 #pragma unroll
         for (int m = 0; m < MEQN; m++) {
-            double f[4];
+            double fh[4], fl[4], f[4];
+            cell_faces(a, T, i, j, ci, cj, m, ax, ay, fh, fl);
 #pragma unroll
-            for (int k = 0; k < 4; k++) f[k] = add(mul(th[k], sub(fh[k][m], fl[k][m])), fl[k][m]);
+            for (int k = 0; k < 4; k++) f[k] = add(mul(th[k], sub(fh[k], fl[k])), fl[k]);
             // FinSolveLxW.cpp:145-148
-            double v = sub(qc[m], mul(dtdx, sub(f[1], f[0])));
+            double v = sub(T.q[m][ci + 1][cj + 1], mul(dtdx, sub(f[1], f[0])));
             v = sub(v, mul(dtdy, sub(f[3], f[2])));
             qn[m] = v;
-            a.qout[m * a.plane + (size_t(i) * my + j)] = v;
+            a.qout[m * a.plane + c] = v;
         }
         // GlobalWaveSpd.cpp:71-76 on the new state
         const double rho = qn[0];
@@ -253,7 +334,7 @@ __global__ void __launch_bounds__(128) k_mpp_update(const MppArgs a)
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        for (int w = 1; w < 4; w++) {
+        for (int w = 1; w < NT / 32; w++) {
             sx = Max(sx, red[0][w]);
             sy = Max(sy, red[1][w]);
         }
