@@ -22,6 +22,27 @@
 namespace fin {
 namespace ind {
 
+// Rows 0 and 4, and row 1, of the left projection for a pair of vectors.
+__device__ __forceinline__ void left04_x2(const Euler::Eig<float>& e, const Euler::Rows<float>& r, const f2* v, f2& w0,
+                                          f2& w4)
+{
+    // ct = c (v4 - u2 v2 - u3 v3); w0 = (a0 v1 + b0 v0 + ct) inv_cd; w4 = (a4 v1 + b4 v0 + ct) inv_cd
+    const f2 ct = f2_mul(f2_splat(e.cl),
+                         f2_fma(f2_splat(-e.u3), v[3], f2_fma(f2_splat(-e.u2), v[2], v[4])));
+    w0 = f2_mul(f2_add(f2_fma(f2_splat(r.a0), v[1], f2_mul(f2_splat(r.b0), v[0])), ct), f2_splat(e.inv_cd));
+    w4 = f2_mul(f2_add(f2_fma(f2_splat(r.a4), v[1], f2_mul(f2_splat(r.b4), v[0])), ct), f2_splat(e.inv_cd));
+}
+__device__ __forceinline__ f2 left1_x2(const Euler::Eig<float>& e, const Euler::Rows<float>& r, const f2* v)
+{
+    // (e1 v0 + u1 v1 + u2 v2 + u3 v3 - v4) inv_d2
+    f2 a = f2_mul(f2_splat(r.e1), v[0]);
+    a = f2_fma(f2_splat(e.u1), v[1], a);
+    a = f2_fma(f2_splat(e.u2), v[2], a);
+    a = f2_fma(f2_splat(e.u3), v[3], a);
+    a = f2_fma(f2_splat(-1.0f), v[4], a);
+    return f2_mul(a, f2_splat(e.inv_d2));
+}
+
 constexpr int NFEAT = 20;
 constexpr float FEAT_FLOOR = 1e-3f;
 

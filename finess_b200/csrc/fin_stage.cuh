@@ -48,7 +48,6 @@
 #include "fin_device.cuh"
 #include "fin_tc.cuh"
 #include "fin_weno_face.cuh"
-#include <type_traits>
 
 namespace fin {
 
@@ -370,11 +369,7 @@ __device__ __forceinline__ R stage_face(const StageArgs& a, const StageSmem<R, C
     Qa[2] = R(0.5) * (qb[CT * PQ] + qb[CT * PQ - QSTR]);
     Qa[3] = R(0.5) * (qb[3 * PQ] + qb[3 * PQ - QSTR]);
     Qa[4] = R(0.5) * (qb[4 * PQ] + qb[4 * PQ - QSTR]);
-    constexpr bool X2 = sizeof(R) == 4 && (P2 || VER == FIN_WENO_FD);   // FP32: f32x2 pairs
-    typename std::conditional<X2, Euler::Eig<R>, Euler::Face<R>>::type ev;
-    R ir;
-    if constexpr (X2) { ev = Euler::eig(gamma, Qa); ir = rcp(Qa[0]); }
-    else { ev = Euler::face(gamma, Qa); ir = ev.ir; }
+    const Euler::Face<R> ev = Euler::face(gamma, Qa);
     // SetWaveSpd.cpp:39-68 from the two cells' u_n, p, c (nmag = 1) and
     // the LLF alpha of ConstructL.cpp:172-174.
     R alpha;
@@ -385,7 +380,7 @@ __device__ __forceinline__ R stage_face(const StageArgs& a, const StageSmem<R, C
         const R cl = pb[3 * PQ - QSTR], cr = pb[3 * PQ];
         const R ua = R(0.5) * (unl + unr);
         const R pa = R(0.5) * (pl + pr);
-        const R ca = sqrt_fast(fabs(gamma * pa * ir));
+        const R ca = sqrt_fast(fabs(gamma * pa * ev.ir));
         if (pa < R(0) || Qa[0] < R(0)) neg = true;
         const R s1 = Min(unl - cl, ua - ca);
         const R s2 = Max(unr + cr, ua + ca);
@@ -404,16 +399,17 @@ __device__ __forceinline__ R stage_face(const StageArgs& a, const StageSmem<R, C
     // 0..4; gm the same with -l_alpha, points 5..1 (ConstructL.cpp:179-185).
     const R lah = R(0.5) * Par<R>::ascale(a) * alpha;
     R fh[MEQN];
-    if constexpr (X2) {
-        // the split pairs and the paired reconstructions of weno_char_flux_x2
-        auto pt = [&](int s, float* q, float* f) {
+    if constexpr (sizeof(R) == 4) {
+        auto pt = [&](int s, f2* v) {
             const int oq = (s - 3) * QSTR, of = (s - 3) * FSTR;
-            q[0] = qb[oq]; q[1] = qb[CN * PQ + oq]; q[2] = qb[CT * PQ + oq]; q[3] = qb[3 * PQ + oq];
-            q[4] = qb[4 * PQ + oq];
-            f[0] = fb[of]; f[1] = fb[CN * FP + of]; f[2] = fb[CT * FP + of]; f[3] = fb[3 * FP + of];
-            f[4] = fb[4 * FP + of];
+            v[0] = f2_make(fb[of], qb[oq]);
+            v[1] = f2_make(fb[CN * FP + of], qb[CN * PQ + oq]);
+            v[2] = f2_make(fb[CT * FP + of], qb[CT * PQ + oq]);
+            v[3] = f2_make(fb[3 * FP + of], qb[3 * PQ + oq]);
+            v[4] = f2_make(fb[4 * FP + of], qb[4 * PQ + oq]);
         };
-        weno_char_flux_x2<VER>(ev, lah, pt, eps, fh);
+        auto slot = [&](int m) -> R& { return out[(m == 1 ? CN : m == 2 ? CT : m) * OP]; };
+        weno_char_flux<VER, P2>(ev, lah, eps, pw, pt, [&](int m, R x) { slot(m) = x; }, [&](int m) { return slot(m); }, fh);
     } else {
         // The reconstructed split values are their upwind points plus
         // corrections (weno5_diff), and R L = I, so the face flux is

@@ -105,40 +105,39 @@ __device__ __forceinline__ void hyb_troubled_face(int w, const float2* fqx, cons
     const int cn = isx ? 1 : 2, ct = isx ? 2 : 1;
     const float2* P0 = isx ? fqx + fi * TJ + fj : fqy + fi * RJ + fj;   // stencil point 0
     const int str = isx ? TJ : 1, pl = isx ? XPL : YPL;
-    auto pt = [&](int s, float* q, float* f) {
+    auto pt = [&](int s, f2* v) {
         const float2* P = P0 + s * str;
-        const float2 v0 = P[0], vn = P[cn * pl], vt = P[ct * pl], vw = P[3 * pl], ve = P[4 * pl];
-        q[0] = v0.y; q[1] = vn.y; q[2] = vt.y; q[3] = vw.y; q[4] = ve.y;
-        f[0] = v0.x; f[1] = vn.x; f[2] = vt.x; f[3] = vw.x; f[4] = ve.x;
+        v[0] = f2_of(P[0]);
+        v[1] = f2_of(P[cn * pl]);
+        v[2] = f2_of(P[ct * pl]);
+        v[3] = f2_of(P[3 * pl]);
+        v[4] = f2_of(P[4 * pl]);
     };
     // face average (ConstructL.cpp:72-77), normal frame
     float Qa[MEQN];
     {
-        float q2[MEQN], q3[MEQN], f2[MEQN], f3[MEQN];
-        pt(2, q2, f2);
-        pt(3, q3, f3);
+        f2 v2[MEQN], v3[MEQN];
+        pt(2, v2);
+        pt(3, v3);
 #pragma unroll
-        for (int m = 0; m < MEQN; m++) Qa[m] = 0.5f * (q3[m] + q2[m]);
+        for (int m = 0; m < MEQN; m++) Qa[m] = 0.5f * (f2_hi(v3[m]) + f2_hi(v2[m]));
     }
-    const typename Euler::Eig<float> ev = Euler::eig(gam, Qa);
+    const Euler::Face<float> ev = Euler::face(gam, Qa);
     const int qb = (H + fi) * RJ + (H + fj), ql = qb - (isx ? RJ : 1);
     const float4 PL = prim4[ql], PR = prim4[qb];
     const float unl = isx ? PL.x : PL.y, unr = isx ? PR.x : PR.y;
     const float ua = 0.5f * (unl + unr), pa = 0.5f * (PL.z + PR.z);
-    const float ca = fsqrt(fabsf(gam * pa * rcp(Qa[0])));
+    const float ca = fsqrt(fabsf(gam * pa * ev.ir));
     const float s1 = Min(unl - PL.w, ua - ca), s2 = Max(unr + PR.w, ua + ca);
     const float alpha = Max(isx ? ag1 : ag2, Max(fabsf(s1), fabsf(s2)));
+    float* const out = (isx ? Fh : Gh) + fi * FP + fj;
+    const int op = isx ? (TI + 1) * FP : TI * FP;
+    auto slot = [&](int m) -> float& { return out[(m == 1 ? cn : m == 2 ? ct : m) * op]; };
     float fh[MEQN];
-    if constexpr (P2 || VER == FIN_WENO_FD) weno_char_flux_x2<VER>(ev, ash * alpha, pt, eps, fh);   // f32x2 pairs
-    else weno_char_flux<float, VER, P2>(ev, ash * alpha, eps, pw, pt, fh);
-    if (isx) {
+    weno_char_flux<VER, P2>(ev, ash * alpha, eps, pw, pt, [&](int m, float x) { slot(m) = x; },
+                            [&](int m) { return slot(m); }, fh);
 #pragma unroll
-        for (int m = 0; m < MEQN; m++) Fh[m * (TI + 1) * FP + fi * FP + fj] = fh[m];
-    } else {
-        const float o[MEQN] = {fh[0], fh[2], fh[1], fh[3], fh[4]};
-#pragma unroll
-        for (int m = 0; m < MEQN; m++) Gh[m * TI * FP + fi * FP + fj] = o[m];
-    }
+    for (int m = 0; m < MEQN; m++) slot(m) = fh[m];
 }
 
 // One stage on the cell tile (i0, j0) of the state a describes.  With a.tma
