@@ -403,14 +403,18 @@ k_stage_batch(const BProb* pr, const int* act, const long long* tile0, const int
 }
 
 // One hybrid stage over the problems of a queue (stage_hyb_tile, the body of
-// k_stage_hyb, with the tile staged by loads: args have tma = 0).
+// k_stage_hyb; tiles of problems with tensor maps are staged by TMA on the
+// successive phases of one mbarrier).
 template <int VER, bool P2, class Cfg>
 __global__ void __launch_bounds__(Cfg::NT, FIN_HYB_CTAS)
 k_stage_hyb_batch(const BProb* pr, const int* act, const long long* tile0, const int* nact, const StageArgs* args,
                   unsigned long long* queue)
 {
+    uint32_t phase = 0;
+    hyb_mbar_init<Cfg>();
     walk_queue<Cfg::TI, Cfg::TJ>(pr, act, tile0, nact, queue, [&](int p, int i0, int j0) {
-        stage_hyb_tile<VER, P2, Cfg>(args[p], i0, j0);
+        stage_hyb_tile<VER, P2, Cfg>(args[p], i0, j0, phase);
+        tc::fence_smem_to_async();   // the next tile's copy lands where this tile's face fluxes were stored
         return true;
     });
 }

@@ -45,6 +45,24 @@ __device__ __forceinline__ void atomic_max_nonneg(double* addr, double v)
 template <class R> __host__ __device__ __forceinline__ R Max(R a, R b) { return a > b ? a : b; }
 template <class R> __host__ __device__ __forceinline__ R Min(R a, R b) { return a < b ? a : b; }
 
+// Maximum and minimum that give NaN when either operand is NaN: one FP32
+// instruction where the comparison forms above take two.  Used for wave
+// speeds, where a NaN comes from a state that the non-finite check reports.
+__device__ __forceinline__ float MaxN(float a, float b)
+{
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float MinN(float a, float b)
+{
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ double MaxN(double a, double b) { return Max(a, b); }
+__device__ __forceinline__ double MinN(double a, double b) { return Min(a, b); }
+
 // Reciprocal by one third-order step from the hardware approximation (PTX
 // rcp.approx.ftz): with e = 1 - x r, 1/x = r (1 + e + e^2 + ...), and the
 // series cut after e^2 cubes the approximation's relative error (about 2^-20)

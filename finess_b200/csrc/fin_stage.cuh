@@ -296,6 +296,11 @@ __device__ __forceinline__ double warp_max_nonneg(double v)
     return __hiloint2double(int(mh), int(ml));
 }
 
+__device__ __forceinline__ float warp_max_nonneg(float v)
+{
+    return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));
+}
+
 // Shared-memory arrays of a stage tile.
 template <class R, class Cfg>
 struct StageSmem {
@@ -382,9 +387,9 @@ __device__ __forceinline__ R stage_face(const StageArgs& a, const StageSmem<R, C
         const R pa = R(0.5) * (pl + pr);
         const R ca = sqrt_fast(fabs(gamma * pa * ev.ir));
         if (pa < R(0) || Qa[0] < R(0)) neg = true;
-        const R s1 = Min(unl - cl, ua - ca);
-        const R s2 = Max(unr + cr, ua + ca);
-        alpha = Max(ag, Max(fabs(s1), fabs(s2)));
+        const R s1 = MinN(unl - cl, ua - ca);
+        const R s2 = MaxN(unr + cr, ua + ca);
+        alpha = MaxN(ag, MaxN(R(fabs(s1)), R(fabs(s2))));
     }
     // GetCFL's Max skips NaN entries (Max(NaN, c) = c), so only finite face
     // speeds enter the CFL maximum.
@@ -631,7 +636,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const int i0, con
     __syncthreads();
 
     // ---- phase 2: one thread per face, x faces then y faces ----
-    double smax_x = 0.0, smax_y = 0.0;
+    R smax_x = R(0), smax_y = R(0);
     bool neg = false, nonfinite = false;
     {
         const R ag1 = a.alpha_in ? R(a.alpha_in[0]) : R(0);
@@ -640,7 +645,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const int i0, con
             bool in_cfl;
             const R al = stage_face<R, VER, P2, Cfg, FG, true>(a, S, k, i0, j0, ag1, neg, in_cfl);
             if (!(al <= R(1e30))) nonfinite = true;
-            else if (in_cfl) smax_x = Max(smax_x, double(al));
+            else if (in_cfl) smax_x = MaxN(smax_x, al);
         }
         const R ag2 = a.alpha_in ? R(a.alpha_in[1]) : R(0);
 #pragma unroll 1
@@ -648,14 +653,14 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const int i0, con
             bool in_cfl;
             const R al = stage_face<R, VER, P2, Cfg, FG, false>(a, S, k, i0, j0, ag2, neg, in_cfl);
             if (!(al <= R(1e30))) nonfinite = true;
-            else if (in_cfl) smax_y = Max(smax_y, double(al));
+            else if (in_cfl) smax_y = MaxN(smax_y, al);
         }
     }
     if (OPND) asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
 
     // ---- phase 3: flux difference, stage update, next-stage wave speed ----
-    double cs_x = 0.0, cs_y = 0.0;
+    R cs_x = R(0), cs_y = R(0);
     const double gam = a.gamma;
     for (int c = tid; c < ((FG && a.flux_only) ? 0 : TI * TJ); c += NT) {
         const int ci = c / TJ, cj = c - ci * TJ;
@@ -709,21 +714,21 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const int i0, con
             // it in FP32.
             const R qx[MEQN] = {R(qn[0]), R(qn[1]), R(qn[2]), R(qn[3]), R(qn[4])};
             const typename Euler::Cell<R> w = Euler::cell(R(gam), qx);
-            const double sx = double(fabs(w.un) + w.c);
-            const double sy = double(fabs(qx[2] * rcp(qx[0])) + w.c);
-            if (!(sx <= 1e300) || !(sy <= 1e300)) nonfinite = true;
-            if (sx <= 1e300) cs_x = Max(cs_x, sx);
-            if (sy <= 1e300) cs_y = Max(cs_y, sy);
+            const R sx = fabs(w.un) + w.c, sy = fabs(qx[2] * rcp(qx[0])) + w.c;
+            const R big = sizeof(R) == 8 ? R(1e300) : R(3e38f);
+            if (!(sx <= big) || !(sy <= big)) nonfinite = true;
+            if (sx <= big) cs_x = MaxN(cs_x, sx);
+            if (sy <= big) cs_y = MaxN(cs_y, sy);
         }
     }
 
     // ---- block reductions of the four maxima, one atomic each ----
     // Non-finite speeds were flagged per value above (a NaN does not survive
     // Max(NaN, b) = b), so the reduction only sees finite ones.
-    const double v4[4] = {smax_x, smax_y, cs_x, cs_y};
+    const R v4[4] = {smax_x, smax_y, cs_x, cs_y};
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-        const double v = warp_max_nonneg(v4[k] <= 1e300 ? v4[k] : 0.0);
+        const double v = double(warp_max_nonneg(v4[k]));
         if ((tid & 31) == 0) S.red[(tid >> 5) * 4 + k] = v;
     }
     if (neg) atomicOr(a.status, 2u);

@@ -5,7 +5,13 @@
 //     linear FD5 flux in its component-wise 6-point form (linear_face), which
 //     equals the reference's characteristic FD5 path (WenoReconstruct_FD5,
 //     lib/WenoReconstruct.cpp:580-616) because the reconstruction is linear;
-//   * troubled faces: the full characteristic WENO flux (weno_char_flux).
+//   * troubled faces: the full characteristic WENO flux (weno_char_flux), x
+//     and y faces from lists of their own, so that every stencil address is a
+//     constant offset; pass A leaves each face's speed in its flux slot.
+//     Measured (B200, eight steps at 4096^2 with a third of the faces
+//     troubled): 35.1 -> 31.0 ms against one list with strides chosen at run
+//     time and the speed computed twice (spills 118 -> 8 bytes a thread, and
+//     one-instruction maxima).
 // Layout and schedule, for B200:
 //   * one TI x TJ tile per CTA, three CTAs (24 warps) per SM;
 //   * q_in's tile + halo arrives by one TMA copy (tiles clear of the domain
@@ -54,8 +60,8 @@ struct HybSmem {
     static constexpr size_t EBUF = Cfg::pad128(SHARE ? STG + Cfg::STG_BYTES : FH + FHGH);   // double [M][TI][TJ]
     static constexpr size_t RED = SHARE ? EBUF : EBUF + Cfg::ABUF_BYTES;               // double [NT/32][4]
     static constexpr size_t MASK = RED + size_t(NT / 32) * 4 * 8;                       // unsigned [FXR + FYR]
-    static constexpr size_t NTRB = MASK + 4 * size_t(Cfg::FXR + Cfg::FYR);              // int
-    static constexpr size_t TLIST = NTRB + 4;                                            // short [NFX + NFY]
+    static constexpr size_t NTRB = MASK + 4 * size_t(Cfg::FXR + Cfg::FYR);              // int [2]
+    static constexpr size_t TLIST = NTRB + 8;                                            // short [NFX + NFY]
     static constexpr size_t MBAR = (TLIST + 2 * size_t(Cfg::NFX + Cfg::NFY) + 7) / 8 * 8;   // uint64
     static constexpr size_t BYTES = MBAR + 8;
     static_assert(!SHARE || FHGH <= Cfg::STG_BYTES, "the face fluxes fit the staging tile");
@@ -88,23 +94,21 @@ __device__ __forceinline__ float linear_face2(const float2* P, int str, float la
 #endif
 }
 
-// Pass B of k_stage_hyb for one troubled face w (work-list index): the
-// LLF speed again, the face-average eigensystem and the full characteristic
-// WENO flux, stored into Fh / Gh.
-template <int VER, bool P2, class Cfg>
-__device__ __forceinline__ void hyb_troubled_face(int w, const float2* fqx, const float2* fqy, const float4* prim4,
-                                               float* Fh, float* Gh, float gam, float eps, float pw, float ash,
-                                               float ag1, float ag2)
+// Pass B of k_stage_hyb for one troubled face of direction x (ISX) or y, w
+// = fi TJ + fj or fi (TJ+1) + fj: the face-average eigensystem and the full
+// characteristic WENO flux, stored into Fh / Gh, where pass A has left the
+// face's LLF speed in the slot of component 0.
+template <int VER, bool P2, class Cfg, bool isx>
+__device__ __forceinline__ void hyb_troubled_face(int w, const float2* fqx, const float2* fqy, float* Fh, float* Gh,
+                                                  float gam, float eps, float pw, float ash)
 {
-    constexpr int TI = Cfg::TI, TJ = Cfg::TJ, H = Cfg::H, RI = Cfg::RI, RJ = Cfg::RJ;
+    constexpr int TI = Cfg::TI, TJ = Cfg::TJ, RI = Cfg::RI, RJ = Cfg::RJ;
     constexpr int XPL = RI * TJ, YPL = TI * RJ, FP = HybSmem<Cfg>::FP;
-    const bool isx = w < Cfg::NFX;
-    int fi, fj;
-    if (isx) { fi = w / TJ; fj = w - fi * TJ; }
-    else { const int v = w - Cfg::NFX; fi = v / (TJ + 1); fj = v - fi * (TJ + 1); }
-    const int cn = isx ? 1 : 2, ct = isx ? 2 : 1;
+    constexpr int NJ = isx ? TJ : TJ + 1;
+    const int fi = w / NJ, fj = w - fi * NJ;
+    constexpr int cn = isx ? 1 : 2, ct = isx ? 2 : 1;
     const float2* P0 = isx ? fqx + fi * TJ + fj : fqy + fi * RJ + fj;   // stencil point 0
-    const int str = isx ? TJ : 1, pl = isx ? XPL : YPL;
+    constexpr int str = isx ? TJ : 1, pl = isx ? XPL : YPL;
     auto pt = [&](int s, f2* v) {
         const float2* P = P0 + s * str;
         v[0] = f2_of(P[0]);
@@ -123,15 +127,9 @@ __device__ __forceinline__ void hyb_troubled_face(int w, const float2* fqx, cons
         for (int m = 0; m < MEQN; m++) Qa[m] = 0.5f * (f2_hi(v3[m]) + f2_hi(v2[m]));
     }
     const Euler::Face<float> ev = Euler::face(gam, Qa);
-    const int qb = (H + fi) * RJ + (H + fj), ql = qb - (isx ? RJ : 1);
-    const float4 PL = prim4[ql], PR = prim4[qb];
-    const float unl = isx ? PL.x : PL.y, unr = isx ? PR.x : PR.y;
-    const float ua = 0.5f * (unl + unr), pa = 0.5f * (PL.z + PR.z);
-    const float ca = fsqrt(fabsf(gam * pa * ev.ir));
-    const float s1 = Min(unl - PL.w, ua - ca), s2 = Max(unr + PR.w, ua + ca);
-    const float alpha = Max(isx ? ag1 : ag2, Max(fabsf(s1), fabsf(s2)));
     float* const out = (isx ? Fh : Gh) + fi * FP + fj;
-    const int op = isx ? (TI + 1) * FP : TI * FP;
+    constexpr int op = isx ? (TI + 1) * FP : TI * FP;
+    const float alpha = out[0];
     auto slot = [&](int m) -> float& { return out[(m == 1 ? cn : m == 2 ? ct : m) * op]; };
     float fh[MEQN];
     weno_char_flux<VER, P2>(ev, ash * alpha, eps, pw, pt, [&](int m, float x) { slot(m) = x; },
@@ -140,12 +138,26 @@ __device__ __forceinline__ void hyb_troubled_face(int w, const float2* fqx, cons
     for (int m = 0; m < MEQN; m++) slot(m) = fh[m];
 }
 
-// One stage on the cell tile (i0, j0) of the state a describes.  With a.tma
-// the tile's copies run on an mbarrier initialised here, so a CTA calls this
-// once (k_stage_hyb); a persistent caller that walks several tiles passes
-// a.tma = 0 and separates the calls by a barrier.
+// The mbarrier of a CTA's tile copies, initialised once per CTA before the
+// first stage_hyb_tile (which has a CTA barrier between this and the first
+// wait): an mbarrier may not be initialised again while it is valid, so the
+// tiles of a persistent CTA use its successive phases.
+template <class Cfg>
+__device__ __forceinline__ void hyb_mbar_init()
+{
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    if (threadIdx.x == 0) {
+        tc::mbar_init(reinterpret_cast<uint64_t*>(smem_raw + HybSmem<Cfg>::MBAR), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+}
+
+// One stage on the cell tile (i0, j0) of the state a describes.  phase is the
+// parity of the mbarrier phase that the next tile copy completes (0 at first;
+// the same in every thread).  A persistent caller separates the calls by a
+// barrier.
 template <int VER, bool P2, class Cfg>
-__device__ __forceinline__ void stage_hyb_tile(const StageArgs& a, const int i0, const int j0)
+__device__ __forceinline__ void stage_hyb_tile(const StageArgs& a, const int i0, const int j0, uint32_t& phase)
 {
     using R = float;
     using L = HybSmem<Cfg>;
@@ -187,8 +199,6 @@ __device__ __forceinline__ void stage_hyb_tile(const StageArgs& a, const int i0,
         const CUtensorMap* tme = a.gtm_A ? a.gtm_A : &a.tm_A;
         if (a.gtm_in) tc::tensormap_acquire(a.gtm_in);
         if (ext && a.gtm_A) tc::tensormap_acquire(a.gtm_A);
-        tc::mbar_init(mbq, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         tc::mbar_expect_tx(mbq, uint32_t(Cfg::STG_BYTES + (ext && !L::SHARE ? Cfg::ABUF_BYTES : 0)));
         tc::tma_load_3d(stg, tmi, j0 - 4, i0 - H, 0, mbq);
         if (ext && !L::SHARE) tc::tma_load_3d(ebuf, tme, j0, i0, 0, mbq);
@@ -220,13 +230,16 @@ __device__ __forceinline__ void stage_hyb_tile(const StageArgs& a, const int i0,
             fym[tid - 32] = msk | (msk >> 1) | (msk >> 2);
         }
     }
-    if (tid == 0) *ntrb = 0;
+    if (tid < 2) ntrb[tid] = 0;
     __syncthreads();
-    if (tt && !tc::mbar_wait(mbq, 0, 1u << 24)) {
-        // the copy did not land in time: report it, and give it one more
-        // bounded wait before the shared memory is read or released
-        atomicOr(a.status, 8u);
-        tc::mbar_wait(mbq, 0, 1u << 24);
+    if (tt) {
+        if (!tc::mbar_wait(mbq, phase, 1u << 20)) {
+            // the copy did not land in time: report it, and give it one more
+            // bounded wait before the shared memory is read or released
+            atomicOr(a.status, 8u);
+            tc::mbar_wait(mbq, phase, 1u << 20);
+        }
+        phase ^= 1u;
     }
     {
         // ---- phase 1: per cell of the cross region: narrow to FP32,
@@ -286,43 +299,45 @@ __device__ __forceinline__ void stage_hyb_tile(const StageArgs& a, const int i0,
             const float ua = 0.5f * (unl + unr), pa = 0.5f * (PL.z + PR.z);
             const float ca = fsqrt(fabsf(gam * pa * rcp(rho)));
             if (pa < 0.0f || rho < 0.0f) neg = true;
-            const float s1 = Min(unl - PL.w, ua - ca), s2 = Max(unr + PR.w, ua + ca);
-            const float alpha = Max(isx ? ag1 : ag2, Max(fabsf(s1), fabsf(s2)));
+            const float s1 = MinN(unl - PL.w, ua - ca), s2 = MaxN(unr + PR.w, ua + ca);
+            const float alpha = MaxN(isx ? ag1 : ag2, MaxN(fabsf(s1), fabsf(s2)));
             if (!(alpha <= 1e30f)) nonfinite = true;
             const unsigned* fm = isx ? fxm : fym;
             const bool trb = (((fm[fi] | fm[fi + 1] | fm[fi + 2]) >> fj) & 1u) != 0;
             if (i0 + fi < mx && j0 + fj < my && alpha <= 1e30f) {
-                if (isx) smax_x = Max(smax_x, alpha);
-                else smax_y = Max(smax_y, alpha);
+                if (isx) smax_x = MaxN(smax_x, alpha);
+                else smax_y = MaxN(smax_y, alpha);
             }
-            if (!trb) {
+            float* dst = (isx ? Fh : Gh) + fi * FP + fj;
+            if (trb) {
+                dst[0] = alpha;   // for pass B
+            } else {
                 const float lah = ash * alpha;
-                float* dst = (isx ? Fh : Gh) + fi * FP + fj;
                 constexpr int dplane = isx ? (TI + 1) * FP : TI * FP;
 #pragma unroll
                 for (int m = 0; m < MEQN; m++) dst[m * dplane] = linear_face2(P + m * pl, str, lah);
             }
             return trb;
         };
-        auto append = [&](bool push, int w) {
+        auto append = [&](bool push, int w, int* count, short* list) {
             const unsigned bal = __ballot_sync(0xffffffffu, push);
             if (bal) {
                 int base = 0;
-                if (lane == __ffs(bal) - 1) base = atomicAdd(ntrb, __popc(bal));
+                if (lane == __ffs(bal) - 1) base = atomicAdd(count, __popc(bal));
                 base = __shfl_sync(0xffffffffu, base, __ffs(bal) - 1);
-                if (push) tlist[base + __popc(bal & ((1u << lane) - 1u))] = short(w);
+                if (push) list[base + __popc(bal & ((1u << lane) - 1u))] = short(w);
             }
         };
         // One face per thread, x faces then y faces: a half-warp takes 16
         // faces of one row (it reads one row of the pairs and primitives),
         // the two half-warps of a warp rows 8 apart (the flux stores fall in
         // opposite bank halves); the last warp of y faces takes row 7 and
-        // the last column.  The list holds face indices (fi (TJ+1) + fj for
-        // y faces after the NFX x faces, fi TJ + fj for x faces).
+        // the last column.  The two lists hold face indices (fi TJ + fj for x
+        // faces, fi (TJ+1) + fj for y faces).
         {
             const int w = tid, fi = (w >> 5) + ((w >> 1) & 8), fj = w & 15;
             const bool push = face_a(std::true_type{}, fi, fj);
-            append(push, fi * TJ + fj);
+            append(push, fi * TJ + fj, ntrb, tlist);
         }
         {
             const int v = tid, wv = v >> 5, ln = v & 31;
@@ -332,16 +347,23 @@ __device__ __forceinline__ void stage_hyb_tile(const StageArgs& a, const int i0,
             else { fi = ln - 16; fj = TJ; }
             bool push = false;
             if (v < Cfg::NFY) push = face_a(std::false_type{}, fi, fj);
-            append(push, Cfg::NFX + fi * (TJ + 1) + fj);
+            append(push, fi * (TJ + 1) + fj, ntrb + 1, tlist + Cfg::NFX);
         }
         __syncthreads();
         // ---- phase 2, pass B: full characteristic WENO on the listed faces ----
         {
-            const int nt = *ntrb;
-            const float agx[2] = {ag1, ag2};
+            // x faces, then y faces from the next whole warp on, so that a
+            // warp's faces share their compile-time strides
+            const int nx = ntrb[0], ny = ntrb[1], y0 = (nx + 31) & ~31;
 #pragma unroll 1
-            for (int k = tid; k < nt; k += NT)
-                hyb_troubled_face<VER, P2, Cfg>(tlist[k], fqx, fqy, prim4, Fh, Gh, gam, eps, pw, ash, agx[0], agx[1]);
+            for (int k = tid; k < y0 + ny; k += NT) {
+                if (k < y0) {
+                    if (k < nx)
+                        hyb_troubled_face<VER, P2, Cfg, true>(tlist[k], fqx, fqy, Fh, Gh, gam, eps, pw, ash);
+                } else {
+                    hyb_troubled_face<VER, P2, Cfg, false>(tlist[Cfg::NFX + k - y0], fqx, fqy, Fh, Gh, gam, eps, pw, ash);
+                }
+            }
         }
         __syncthreads();
         // ---- phase 3: flux difference (ConstructL.cpp:396-398), update
@@ -399,8 +421,8 @@ __device__ __forceinline__ void stage_hyb_tile(const StageArgs& a, const int i0,
                     const float cc = fsqrt(fabsf(gam * press * ir));
                     const float sx = fabsf(u1) + cc, sy = fabsf(u2) + cc;
                     if (!(sx <= 1e30f) || !(sy <= 1e30f)) nonfinite = true;
-                    if (sx <= 1e30f) csx = Max(csx, sx);
-                    if (sy <= 1e30f) csy = Max(csy, sy);
+                    if (sx <= 1e30f) csx = MaxN(csx, sx);
+                    if (sy <= 1e30f) csy = MaxN(csy, sy);
                 }
             }
         }
@@ -408,17 +430,11 @@ __device__ __forceinline__ void stage_hyb_tile(const StageArgs& a, const int i0,
 
     // ---- block reductions of the four maxima (FP32 values, reduced in
     // FP32), one atomic each ----
-    float v4[4] = {smax_x, smax_y, csx, csy};
+    const float v4[4] = {smax_x, smax_y, csx, csy};
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-        float v = v4[k] <= 1e30f ? v4[k] : 0.0f;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v = Max(v, __shfl_xor_sync(0xffffffffu, v, o));
-        v4[k] = v;
-    }
-    if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k < 4; k++) red[(tid >> 5) * 4 + k] = double(v4[k]);
+        const float v = warp_max_nonneg(v4[k]);
+        if (lane == 0) red[(tid >> 5) * 4 + k] = double(v);
     }
     if (neg) atomicOr(a.status, 2u);
     if (nonfinite) atomicOr(a.status, 1u);
@@ -437,7 +453,9 @@ __global__ void __launch_bounds__(Cfg::NT, FIN_HYB_CTAS) k_stage_hyb(const __gri
 {
     const int ntj = (a.my + Cfg::TJ - 1) / Cfg::TJ;
     const int t = blockIdx.x;
-    stage_hyb_tile<VER, P2, Cfg>(a, (t / ntj) * Cfg::TI, (t % ntj) * Cfg::TJ);
+    uint32_t phase = 0;
+    hyb_mbar_init<Cfg>();
+    stage_hyb_tile<VER, P2, Cfg>(a, (t / ntj) * Cfg::TI, (t % ntj) * Cfg::TJ, phase);
 }
 
 }  // namespace fin
