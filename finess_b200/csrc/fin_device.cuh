@@ -489,10 +489,9 @@ __device__ __forceinline__ R weno5(const R* u, R eps, R pw)
 __device__ __forceinline__ f2 f2_splat(float a) { return f2_make(a, a); }
 // The two corrections (weno5_diff) of a face's split in FP32 as f32x2 pairs
 // (low lane gp, high lane gm), with power 2 or the linear FD5 weights; the
-// weight normalisation's maxima and the reciprocals per lane.  Returns their
-// sum.
+// weight normalisation's maxima and the reciprocals per lane.
 template <int VER>
-__device__ __forceinline__ float weno5_diff_x2(f2 d1, f2 d2, f2 d3, f2 d4, float eps4)
+__device__ __forceinline__ f2 weno5_pair_x2(f2 d1, f2 d2, f2 d3, f2 d4, float eps4)
 {
     const f2 k3 = f2_splat(3.0f), m3 = f2_splat(-3.0f);
     const f2 s0 = f2_fma(k3, d2, f2_mul(f2_splat(-1.0f), d1)), s2 = f2_fma(m3, d3, d4);
@@ -529,6 +528,13 @@ __device__ __forceinline__ float weno5_diff_x2(f2 d1, f2 d2, f2 d3, f2 d4, float
         const f2 den = f2_add(f2_add(w0, w1), w2);
         r = f2_mul(num, f2_make(rcp(f2_lo(den)), rcp(f2_hi(den))));
     }
+    return r;
+}
+// Their sum.
+template <int VER>
+__device__ __forceinline__ float weno5_diff_x2(f2 d1, f2 d2, f2 d3, f2 d4, float eps4)
+{
+    const f2 r = weno5_pair_x2<VER>(d1, d2, d3, d4, eps4);
     return f2_lo(r) + f2_hi(r);
 }
 
