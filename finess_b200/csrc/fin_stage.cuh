@@ -41,9 +41,12 @@
 // multiply-adds and moves fell from 17 to 4 % of the instructions, spills
 // from 180 to 70 bytes), load and flux phases in one, the stage operand
 // copied behind the face phase (q_in's own values taken from shared memory)
-// and the warp maxima by two reduce instructions each.  The FP64 pipe is 61 %
-// busy (52 % before).  The same body changes took the FP32 form's step from
-// 1.69 to 1.48 ms (two steps of 4001 x 515).
+// and the warp maxima by two reduce instructions each (FP64 pipe 61 % busy,
+// 52 % before); 7.33 with the upwind part projected with the rest and
+// everything that only the end of a face needs waiting in its flux slots
+// (no spills; the batch form of the kernel, which had spilled 246 bytes, took
+// 134 instead of 153 ms for a batch of 48).  The same body changes took the
+// FP32 form's step from 1.69 to 1.48 ms (two steps of 4001 x 515).
 #pragma once
 #include "fin_device.cuh"
 #include "fin_tc.cuh"
@@ -416,20 +419,17 @@ __device__ __forceinline__ R stage_face(const StageArgs& a, const StageSmem<R, C
         auto slot = [&](int m) -> R& { return out[(m == 1 ? CN : m == 2 ? CT : m) * OP]; };
         weno_char_flux<VER, P2>(ev, lah, eps, pw, pt, [&](int m, R x) { slot(m) = x; }, [&](int m) { return slot(m); }, fh);
     } else {
-        // The reconstructed split values are their upwind points plus
-        // corrections (weno5_diff), and R L = I, so the face flux is
-        //   (v+ of the left cell + v- of the right cell) + R corr / 6:
-        // the first term in conserved variables, parked in the flux slot
-        // (it would hold ten registers through the sweeps), the second
-        // from differences of the projected points.  Fields 0, 4 and 1 in
-        // one sweep of the stencil, then 2 and 3 (all five at once want
-        // more registers than two CTAs per SM leave).
-#pragma unroll
-        for (int m = 0; m < MEQN; m++)
-            out[m * OP] = (fb[m * FP - FSTR] + fb[m * FP]) + lah * (qb[m * PQ - QSTR] - qb[m * PQ]);
+        // Characteristic values as their upwind points (v+ of the left cell
+        // plus v- of the right cell) plus corrections / 6 from differences of
+        // the projected points (weno5_diff).  Fields 0, 4 and 1 in one sweep
+        // of the stencil, then 2 and 3 (all five at once want more registers
+        // than two CTAs per SM leave); what only the end of the face needs
+        // waits in its flux slots.
         R g[MEQN];
-        const R eps4 = R(4) * eps;
+        const R eps4 = R(4) * eps, s6 = R(1) / R(6);
         {
+            out[3 * OP] = ev.c;
+            out[4 * OP] = ev.h;
             R p0[4], p4[4], m0[4], m4[4], p1[4], m1[4];
             R cp0, cp1, cp4, cm0, cm1, cm4;   // the previous point's values
 #pragma unroll
@@ -447,18 +447,20 @@ __device__ __forceinline__ R stage_face(const StageArgs& a, const StageSmem<R, C
                     const R v[MEQN] = {f0 + lah * q0, fn + lah * qn, ft + lah * qt, fw + lah * qw, fe + lah * qe};
                     Euler::left014(ev, v, w0, w1, w4);
                     if (s > 0) { p0[s - 1] = w0 - cp0; p1[s - 1] = w1 - cp1; p4[s - 1] = w4 - cp4; }
+                    if (s == 2) { out[0] = w0; out[OP] = w1; out[2 * OP] = w4; }
                     cp0 = w0; cp1 = w1; cp4 = w4;
                 }
                 if (s > 0) {
                     const R v[MEQN] = {f0 - lah * q0, fn - lah * qn, ft - lah * qt, fw - lah * qw, fe - lah * qe};
                     Euler::left014(ev, v, w0, w1, w4);
                     if (s > 1) { m0[5 - s] = cm0 - w0; m1[5 - s] = cm1 - w1; m4[5 - s] = cm4 - w4; }
+                    if (s == 3) { out[0] += w0; out[OP] += w1; out[2 * OP] += w4; }
                     cm0 = w0; cm1 = w1; cm4 = w4;
                 }
             }
-            g[0] = weno_pair<R, VER, P2>(p0, m0, eps4, pw);
-            g[4] = weno_pair<R, VER, P2>(p4, m4, eps4, pw);
-            g[1] = weno_pair<R, VER, P2>(p1, m1, eps4, pw);
+            g[0] = s6 * weno_pair<R, VER, P2>(p0, m0, eps4, pw) + out[0];
+            g[4] = s6 * weno_pair<R, VER, P2>(p4, m4, eps4, pw) + out[2 * OP];
+            g[1] = s6 * weno_pair<R, VER, P2>(p1, m1, eps4, pw) + out[OP];
         }
         {
             // fields 2 and 3 (rows v_t - u2 v0 and v_w - u3 v0)
@@ -474,25 +476,24 @@ __device__ __forceinline__ R stage_face(const StageArgs& a, const StageSmem<R, C
                     const R v0 = f0 + lah * q0;
                     const R w2 = (ft + lah * qt) - ev.u2 * v0, w3 = (fw + lah * qw) - ev.u3 * v0;
                     if (s > 0) { p2[s - 1] = w2 - cp2; p3[s - 1] = w3 - cp3; }
+                    if (s == 2) { out[0] = w2; out[OP] = w3; }
                     cp2 = w2; cp3 = w3;
                 }
                 if (s > 0) {
                     const R v0 = f0 - lah * q0;
                     const R w2 = (ft - lah * qt) - ev.u2 * v0, w3 = (fw - lah * qw) - ev.u3 * v0;
                     if (s > 1) { m2[5 - s] = cm2 - w2; m3[5 - s] = cm3 - w3; }
+                    if (s == 3) { out[0] += w2; out[OP] += w3; }
                     cm2 = w2; cm3 = w3;
                 }
             }
-            g[2] = weno_pair<R, VER, P2>(p2, m2, eps4, pw);
-            g[3] = weno_pair<R, VER, P2>(p3, m3, eps4, pw);
+            g[2] = s6 * weno_pair<R, VER, P2>(p2, m2, eps4, pw) + out[0];
+            g[3] = s6 * weno_pair<R, VER, P2>(p3, m3, eps4, pw) + out[OP];
         }
-        Euler::right(ev, g, fh);
-        const R s6 = R(1) / R(6);
-        fh[0] = s6 * fh[0] + out[0];
-        fh[1] = s6 * fh[1] + out[CN * OP];
-        fh[2] = s6 * fh[2] + out[CT * OP];
-        fh[3] = s6 * fh[3] + out[3 * OP];
-        fh[4] = s6 * fh[4] + out[4 * OP];
+        Euler::Face<R> er = ev;
+        er.c = out[3 * OP];
+        er.h = out[4 * OP];
+        Euler::right(er, g, fh);
     }
     // Back to (rho, rho u, rho v, rho w, E) and store.
     const R o[MEQN] = {fh[0], fh[CN], fh[CT], fh[3], fh[4]};
