@@ -51,6 +51,8 @@
 #include "fin_device.cuh"
 #include "fin_tc.cuh"
 #include "fin_weno_face.cuh"
+#include "fin_weno_hi.cuh"
+#include <type_traits>
 
 namespace fin {
 
@@ -123,9 +125,10 @@ __device__ __forceinline__ unsigned row_bits(unsigned lo, unsigned hi, int b0)
     return unsigned(((unsigned long long)hi << 32 | lo) >> (b0 & 31));
 }
 
-template <int TI_, int TJ_, int NT_>
+// A tile of TI x TJ cells, NT threads, stencils reaching H cells out.
+template <int TI_, int TJ_, int NT_, int H_ = 3>
 struct TileCfg {
-    static constexpr int TI = TI_, TJ = TJ_, NT = NT_, H = 3;
+    static constexpr int TI = TI_, TJ = TJ_, NT = NT_, H = H_;
     static constexpr int RI = TI + 2 * H, RJ = TJ + 2 * H;
     static constexpr int NFX = (TI + 1) * TJ, NFY = TI * (TJ + 1);
     static constexpr int NPRIM = 4;   // per-cell u, v, p, c of the cross region
@@ -288,6 +291,17 @@ __device__ __forceinline__ R weno_pair(R* dp, R* dm, R eps4, R pw)
     return g;
 }
 
+// A correction of another order, fenced.
+template <int ORDER, int VER, bool P2>
+__device__ __forceinline__ double hi_fenced(double* d, double eps, double pw)
+{
+#pragma unroll
+    for (int k = 0; k < ORDER - 1; k++) fence(d[k]);
+    double c = hi::correction<ORDER, VER, P2>(d, eps, pw);
+    fence(c);
+    return c;
+}
+
 // Max over a warp of non-negative doubles, as the maximum of their high words
 // and then of the low words that go with it (two warp-reduce instructions
 // instead of five rounds of two shuffles, a compare and two selects).
@@ -333,7 +347,7 @@ struct StageSmem {
 // or y (between columns fj-1 and fj), in registers; the direction is a
 // template parameter, so every stencil address is a constant offset.  Returns
 // the face's LLF speed and whether it enters GetCFL's maximum in *in_cfl.
-template <class R, int VER, bool P2, class Cfg, bool FG, bool ISX>
+template <class R, int VER, bool P2, class Cfg, bool FG, bool ISX, int ORDER>
 __device__ __forceinline__ R stage_face(const StageArgs& a, const StageSmem<R, Cfg>& S, int w, int i0, int j0, R ag,
                                         bool& neg, bool& in_cfl)
 {
@@ -418,6 +432,58 @@ __device__ __forceinline__ R stage_face(const StageArgs& a, const StageSmem<R, C
         };
         auto slot = [&](int m) -> R& { return out[(m == 1 ? CN : m == 2 ? CT : m) * OP]; };
         weno_char_flux<VER, P2>(ev, lah, eps, pw, pt, [&](int m, R x) { slot(m) = x; }, [&](int m) { return slot(m); }, fh);
+    } else if constexpr (ORDER != 5) {
+        // The other orders (FP64): split by split -- gp from v+ at the points
+        // 0 .. ORDER-1, gm from v- at the points ORDER .. 1 -- fields 0, 1 and
+        // 4, then 2 and 3; the fields' sums wait in the face's flux slots.
+        constexpr int NW = ORDER, C = (ORDER - 1) / 2;   // points, the upwind one
+        auto half = [&](auto minus) {
+            constexpr bool M = decltype(minus)::value;
+            const R l = M ? -lah : lah;
+            auto put = [&](int k, R x) {
+                if (M) out[k * OP] += x;
+                else out[k * OP] = x;
+            };
+            {
+                R d0[NW], d1[NW], d4[NW], c0, c1, c4;
+#pragma unroll
+                for (int t = 0; t < NW; t++) {
+                    asm volatile("" ::: "memory");
+                    const int s = M ? NW - t : t, oq = (s - H) * QSTR, of = (s - H) * FSTR;
+                    const R v[MEQN] = {fb[of] + l * qb[oq], fb[CN * FP + of] + l * qb[CN * PQ + oq],
+                                       fb[CT * FP + of] + l * qb[CT * PQ + oq], fb[3 * FP + of] + l * qb[3 * PQ + oq],
+                                       fb[4 * FP + of] + l * qb[4 * PQ + oq]};
+                    R w0, w1, w4;
+                    Euler::left014(ev, v, w0, w1, w4);
+                    if (t > 0) { d0[t - 1] = w0 - c0; d1[t - 1] = w1 - c1; d4[t - 1] = w4 - c4; }
+                    if (t == C) { put(0, w0); put(1, w1); put(4, w4); }
+                    c0 = w0; c1 = w1; c4 = w4;
+                }
+                out[0] += hi_fenced<ORDER, VER, P2>(d0, eps, pw);
+                out[4 * OP] += hi_fenced<ORDER, VER, P2>(d4, eps, pw);
+                out[OP] += hi_fenced<ORDER, VER, P2>(d1, eps, pw);
+            }
+            {
+                R d2[NW], d3[NW], c2, c3;
+#pragma unroll
+                for (int t = 0; t < NW; t++) {
+                    asm volatile("" ::: "memory");
+                    const int s = M ? NW - t : t, oq = (s - H) * QSTR, of = (s - H) * FSTR;
+                    const R v0 = fb[of] + l * qb[oq];
+                    const R w2 = (fb[CT * FP + of] + l * qb[CT * PQ + oq]) - ev.u2 * v0;
+                    const R w3 = (fb[3 * FP + of] + l * qb[3 * PQ + oq]) - ev.u3 * v0;
+                    if (t > 0) { d2[t - 1] = w2 - c2; d3[t - 1] = w3 - c3; }
+                    if (t == C) { put(2, w2); put(3, w3); }
+                    c2 = w2; c3 = w3;
+                }
+                out[2 * OP] += hi_fenced<ORDER, VER, P2>(d2, eps, pw);
+                out[3 * OP] += hi_fenced<ORDER, VER, P2>(d3, eps, pw);
+            }
+        };
+        half(std::false_type{});
+        half(std::true_type{});
+        const R g[MEQN] = {out[0], out[OP], out[2 * OP], out[3 * OP], out[4 * OP]};
+        Euler::right(ev, g, fh);
     } else {
         // Characteristic values as their upwind points (v+ of the left cell
         // plus v- of the right cell) plus corrections / 6 from differences of
@@ -514,7 +580,7 @@ __device__ __forceinline__ R stage_face(const StageArgs& a, const StageSmem<R, C
 }
 
 // One tile (rows i0 .., columns j0 ..) of a stage; the whole CTA takes part.
-template <class R, int VER, bool P2, class Cfg, bool FG = false>
+template <class R, int VER, bool P2, class Cfg, bool FG = false, int ORDER = 5>
 __device__ __forceinline__ void stage_tile(const StageArgs& a, const int i0, const int j0)
 {
     constexpr int TI = Cfg::TI, TJ = Cfg::TJ, NT = Cfg::NT, H = Cfg::H;
@@ -644,7 +710,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const int i0, con
 #pragma unroll 1
         for (int k = tid; k < Cfg::NFX; k += NT) {
             bool in_cfl;
-            const R al = stage_face<R, VER, P2, Cfg, FG, true>(a, S, k, i0, j0, ag1, neg, in_cfl);
+            const R al = stage_face<R, VER, P2, Cfg, FG, true, ORDER>(a, S, k, i0, j0, ag1, neg, in_cfl);
             if (!(al <= R(1e30))) nonfinite = true;
             else if (in_cfl) smax_x = MaxN(smax_x, al);
         }
@@ -652,7 +718,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const int i0, con
 #pragma unroll 1
         for (int k = tid; k < Cfg::NFY; k += NT) {
             bool in_cfl;
-            const R al = stage_face<R, VER, P2, Cfg, FG, false>(a, S, k, i0, j0, ag2, neg, in_cfl);
+            const R al = stage_face<R, VER, P2, Cfg, FG, false, ORDER>(a, S, k, i0, j0, ag2, neg, in_cfl);
             if (!(al <= R(1e30))) nonfinite = true;
             else if (in_cfl) smax_y = MaxN(smax_y, al);
         }
@@ -743,10 +809,11 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const int i0, con
     }
 }
 
-template <class R, int VER, bool P2, class Cfg, bool FG = false>
+template <class R, int VER, bool P2, class Cfg, bool FG = false, int ORDER = 5>
 __global__ void __launch_bounds__(Cfg::NT, MinBlocks<R>::value) k_stage(const __grid_constant__ StageArgs a)
 {
-    stage_tile<R, VER, P2, Cfg, FG>(a, blockIdx.y * Cfg::TI, blockIdx.x * Cfg::TJ);
+    static_assert(ORDER == 5 ? Cfg::H == 3 : Cfg::H == (ORDER + 1) / 2 && sizeof(R) == 8 && !FG, "halo of the stencil");
+    stage_tile<R, VER, P2, Cfg, FG, ORDER>(a, blockIdx.y * Cfg::TI, blockIdx.x * Cfg::TJ);
 }
 
 // GlobalWaveSpd (lib/2d/GlobalWaveSpd.cpp:52-78) on a state already in HBM:

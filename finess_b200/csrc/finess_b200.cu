@@ -24,7 +24,7 @@
 #include "fin_output.h"
 #include "fin_mpp.cuh"
 #include "fin_rk.cuh"
-#include "fin_weno_hi.cuh"
+#include "fin_hi.h"
 #include "fin_sample.cuh"
 
 using namespace fin;
@@ -439,57 +439,14 @@ int launch_stage_hyb(fin_solver* s, const StageArgs& a)
     return set_err(FIN_ERR_ARG, "weno_version");
 }
 
-int grid_blocks(size_t n);
-
-// Spatial orders other than 5 (fin_weno_hi.cuh, FP64): one thread per face
-// into the face-flux arrays, then the flux difference and stage update.
-template <int ORDER, int VER>
-int launch_stage_hi_t(fin_solver* s, const StageArgs& a)
-{
-    const size_t nx = size_t(a.mx + 1) * a.my, ny = size_t(a.mx) * (a.my + 1);
-    if (!s->mpp_fx) CK(cudaMalloc(&s->mpp_fx, MEQN * nx * sizeof(double)));
-    if (!s->mpp_fy) CK(cudaMalloc(&s->mpp_fy, MEQN * ny * sizeof(double)));
-    hi::HiArgs h;
-    memset(&h, 0, sizeof(h));
-    h.q = a.qin;
-    h.plane = a.plane;
-    h.mx = a.mx;
-    h.my = a.my;
-    for (int k = 0; k < 4; k++) h.bc[k] = a.bc[k];
-    h.gamma = a.gamma;
-    h.eps = a.eps;
-    h.pw = a.pw;
-    h.alpha_scaling = a.alpha_scaling;
-    h.alpha_in = a.alpha_in;
-    h.fx = s->mpp_fx;
-    h.fy = s->mpp_fy;
-    h.smax_out = a.smax_out;
-    h.face_alpha_x = a.face_alpha_x;
-    h.face_alpha_y = a.face_alpha_y;
-    h.status = a.status;
-    const size_t nf = nx + ny;
-    hi::k_hi_faces<ORDER, VER><<<unsigned((nf + 127) / 128), 128, 0, s->stream>>>(h);
-    CK(cudaGetLastError());
-    hi::k_hi_update<<<grid_blocks(size_t(a.mx) * a.my), 256, 0, s->stream>>>(s->mpp_fx, s->mpp_fy, a);
-    CK(cudaGetLastError());
-    s->launches += 2;
-    return FIN_OK;
-}
-
+// Spatial orders other than 5 (FP64): instantiated in fin_hi.cu.
 int launch_stage_hi(fin_solver* s, const StageArgs& a)
 {
-    const int v = s->p.weno_version;
-    switch (s->p.space_order) {
-    case 1: return launch_stage_hi_t<1, FIN_WENO_JS>(s, a);
-    case 7:
-        return v == FIN_WENO_Z ? launch_stage_hi_t<7, FIN_WENO_Z>(s, a)
-             : v == FIN_WENO_FD ? launch_stage_hi_t<7, FIN_WENO_FD>(s, a) : launch_stage_hi_t<7, FIN_WENO_JS>(s, a);
-    case 9:
-        return v == FIN_WENO_Z ? launch_stage_hi_t<9, FIN_WENO_Z>(s, a)
-             : v == FIN_WENO_FD ? launch_stage_hi_t<9, FIN_WENO_FD>(s, a) : launch_stage_hi_t<9, FIN_WENO_JS>(s, a);
-    case 11: return launch_stage_hi_t<11, FIN_WENO_JS>(s, a);
-    }
-    return set_err(FIN_ERR_ARG, "Requested WENO Reconstruction not implemented.");
+    const cudaError_t e = fin::hi::launch(s->p.space_order, s->p.weno_version, s->p.power_param == 2.0, a, s->stream);
+    if (e == cudaErrorInvalidValue) return set_err(FIN_ERR_ARG, "Requested WENO Reconstruction not implemented.");
+    CK(e);
+    s->launches++;
+    return FIN_OK;
 }
 
 int launch_stage(fin_solver* s, const StageArgs& a)
