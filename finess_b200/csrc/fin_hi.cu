@@ -11,6 +11,7 @@
 // fused tile with the indicators on differences: LLF 0.84 -> 0.56, JS7 2.93 ->
 // 1.53, Z7 3.30 -> 1.58, FD7 2.11 -> 1.30, JS9 3.58 -> 2.03, Z9 3.98 -> 2.01.
 #include "fin_hi.h"
+#include "fin_pdl.h"
 #include "fin_stage.cuh"
 
 namespace fin {
@@ -29,8 +30,7 @@ cudaError_t launch_t(const StageArgs& a, cudaStream_t stream)
         configured = true;
     }
     const dim3 grid((a.my + Cfg::TJ - 1) / Cfg::TJ, (a.mx + Cfg::TI - 1) / Cfg::TI);
-    kern<<<grid, Cfg::NT, smem, stream>>>(a);
-    return cudaGetLastError();
+    return launch_pdl(kern, grid, dim3(Cfg::NT), smem, stream, a);
 }
 
 template <int ORDER>

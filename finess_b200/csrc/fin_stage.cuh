@@ -131,6 +131,7 @@ struct TileCfg {
     static constexpr int TI = TI_, TJ = TJ_, NT = NT_, H = H_;
     static constexpr int RI = TI + 2 * H, RJ = TJ + 2 * H;
     static constexpr int NFX = (TI + 1) * TJ, NFY = TI * (TJ + 1);
+    static constexpr bool ONE_ROUND = NFX + NFY <= NT;   // a thread per face of the tile
     static constexpr int NPRIM = 4;   // per-cell u, v, p, c of the cross region
     // FP32 faces of a 15 x 16 tile go to threads so that the two half-warps
     // of a warp take face rows 8 apart (XROW8): 8 rows of RJ = 22 words are
@@ -342,6 +343,14 @@ struct StageSmem {
         red = reinterpret_cast<double*>(raw + Cfg::template red_offset<R>());
     }
 };
+
+// The start of a kernel launched by launch_pdl (fin_pdl.h): its successor may
+// be placed, and it waits for its predecessor.
+__device__ __forceinline__ void grid_dependency()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 
 // Flux of face k of direction x (ISX: between rows fi-1 and fi of the tile)
 // or y (between columns fj-1 and fj), in registers; the direction is a
@@ -707,20 +716,29 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const int i0, con
     bool neg = false, nonfinite = false;
     {
         const R ag1 = a.alpha_in ? R(a.alpha_in[0]) : R(0);
-#pragma unroll 1
-        for (int k = tid; k < Cfg::NFX; k += NT) {
+        const R ag2 = a.alpha_in ? R(a.alpha_in[1]) : R(0);
+        auto face_x = [&](int k) {
             bool in_cfl;
             const R al = stage_face<R, VER, P2, Cfg, FG, true, ORDER>(a, S, k, i0, j0, ag1, neg, in_cfl);
             if (!(al <= R(1e30))) nonfinite = true;
             else if (in_cfl) smax_x = MaxN(smax_x, al);
-        }
-        const R ag2 = a.alpha_in ? R(a.alpha_in[1]) : R(0);
-#pragma unroll 1
-        for (int k = tid; k < Cfg::NFY; k += NT) {
+        };
+        auto face_y = [&](int k) {
             bool in_cfl;
             const R al = stage_face<R, VER, P2, Cfg, FG, false, ORDER>(a, S, k, i0, j0, ag2, neg, in_cfl);
             if (!(al <= R(1e30))) nonfinite = true;
             else if (in_cfl) smax_y = MaxN(smax_y, al);
+        };
+        if constexpr (Cfg::ONE_ROUND) {
+            // a thread for every face of the tile, both directions at once
+            static_assert(Cfg::NFX % 32 == 0, "a warp's faces share their direction");
+            if (tid < Cfg::NFX) face_x(tid);
+            else if (tid < Cfg::NFX + Cfg::NFY) face_y(tid - Cfg::NFX);
+        } else {
+#pragma unroll 1
+            for (int k = tid; k < Cfg::NFX; k += NT) face_x(k);
+#pragma unroll 1
+            for (int k = tid; k < Cfg::NFY; k += NT) face_y(k);
         }
     }
     if (OPND) asm volatile("cp.async.wait_all;" ::: "memory");
@@ -810,8 +828,9 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const int i0, con
 }
 
 template <class R, int VER, bool P2, class Cfg, bool FG = false, int ORDER = 5>
-__global__ void __launch_bounds__(Cfg::NT, MinBlocks<R>::value) k_stage(const __grid_constant__ StageArgs a)
+__global__ void __launch_bounds__(Cfg::NT, MinBlocks<R>::value * 256 / Cfg::NT) k_stage(const __grid_constant__ StageArgs a)
 {
+    grid_dependency();
     static_assert(ORDER == 5 ? Cfg::H == 3 : Cfg::H == (ORDER + 1) / 2 && sizeof(R) == 8 && !FG, "halo of the stencil");
     stage_tile<R, VER, P2, Cfg, FG, ORDER>(a, blockIdx.y * Cfg::TI, blockIdx.x * Cfg::TJ);
 }

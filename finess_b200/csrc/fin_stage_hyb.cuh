@@ -455,6 +455,7 @@ __global__ void __launch_bounds__(Cfg::NT, FIN_HYB_CTAS) k_stage_hyb(const __gri
     const int t = blockIdx.x;
     uint32_t phase = 0;
     hyb_mbar_init<Cfg>();
+    grid_dependency();
     stage_hyb_tile<VER, P2, Cfg>(a, (t / ntj) * Cfg::TI, (t % ntj) * Cfg::TJ, phase);
 }
 

@@ -12,6 +12,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <cmath>
+#include <atomic>
 #include <string>
 #include <vector>
 #include <algorithm>
@@ -21,6 +22,7 @@
 #include "fin_intflux.cuh"
 #include "fin_hybrid.cuh"
 #include "fin_tmap.h"
+#include "fin_pdl.h"
 #include "fin_output.h"
 #include "fin_mpp.cuh"
 #include "fin_rk.cuh"
@@ -55,15 +57,22 @@ int set_err(int code, const std::string& msg)
 #endif
 using Cfg = TileCfg<FIN_TILE_TI, FIN_TILE_TJ, FIN_TILE_NT>;
 
-// Reduction slots (doubles) in one device block, reset by one memset per step.
-// The status word (bit 0: non-finite speed or state, bit 1: negative p or rho,
-// bit 2: a tensor-core wait ran out, bit 3: a TMA copy wait ran out, bit 4: a TMA
-// destination was misaligned) sits in slot STATUS so one copy returns it
-// with the maxima.  SMAX_ALT keeps the face-speed maxima of the hybrid attempt
-// while a judge step recomputes with full WENO; DIFF receives the judge's
-// max |q_hybrid - q_full| and max |q_full|.
+// Reduction slots (doubles).  A step's maxima, status word and the global
+// wave speeds of the buffers it writes sit in one of three device blocks that
+// take turns: the step adds into a block that is all zero, q^n's wave speeds
+// stay in the block of the step that made it, and the kernel that publishes a
+// step (k_publish) zeroes the third, so no step begins with a memset.  The
+// status word (bit 0: non-finite speed or state, bit 1: negative p or rho,
+// bit 2: a tensor-core wait ran out, bit 3: a TMA copy wait ran out, bit 4: a
+// TMA destination was misaligned) sits in slot STATUS.  After the blocks:
+// SMAX_ALT keeps the face-speed maxima of the hybrid attempt while a judge step
+// recomputes with full WENO; DIFF receives the judge's max |q_hybrid - q_full|
+// and max |q_full|.  The host's mirror holds one block, SMAX_ALT, DIFF and the
+// number of the step it belongs to (SLOT_SEQ).
 enum { NBUF = 5, SLOT_SMAX = 0, SLOT_ALPHA = 2, SLOT_STATUS = SLOT_ALPHA + 2 * NBUF, SLOT_SMAX_ALT = SLOT_STATUS + 1,
-       SLOT_DIFF = SLOT_SMAX_ALT + 2, NSLOTS = SLOT_DIFF + 2 };
+       SLOT_DIFF = SLOT_SMAX_ALT + 2, NSLOTS = SLOT_DIFF + 2, SLOT_SEQ = NSLOTS, BLOCK = 16, NBLOCK = 3,
+       FIXED = BLOCK * NBLOCK, NDEV = FIXED + 4 };
+static_assert(SLOT_STATUS < BLOCK, "a block holds a step's slots");
 
 }  // namespace
 
@@ -73,9 +82,12 @@ struct fin_solver {
     size_t plane;           // elements per component plane
     double* q[NBUF];        // state buffers (planes); q[cur] holds q^n; q[4] only in the hybrid form
     int cur;                // index of q^n
-    double* slots;          // NSLOTS doubles (+ status word after them)
-    unsigned int* status;
-    double* h_slots;        // pinned mirror
+    double* slots;          // NBLOCK blocks of BLOCK doubles, then SMAX_ALT and DIFF
+    unsigned int* status;   // the status word of block cb
+    double* h_slots;        // pinned mirror (NSLOTS doubles and the step number), written by the device
+    int cb, zb;             // block of the current or last step; the block that is all zero (-1: none)
+    int ablk[NBUF];         // block that holds the global wave speeds of each buffer
+    unsigned long long seq; // steps published
     double* d_aos;          // staging buffer for the reference ghosted layout
     size_t aos_elems;
     double* d_aux;          // second staging / L output buffer (planes)
@@ -210,6 +222,30 @@ __global__ void k_smax_max(const double* smax, int mx, int my, int mbc, double* 
         for (int k = 0; k < nw; k++) v = Max(v, red[threadIdx.x][k]);
         atomic_max_nonneg(out + threadIdx.x, v);
     }
+}
+
+// The end of a step (one warp): its slots to the host's pinned mirror with the
+// step number last, and the next step's block zeroed.  One launch instead of
+// a copy and a stream synchronisation after the step (the host waits on the
+// number) and four or five memsets before the next.  Together with launches
+// that overlap their predecessor's end (fin_pdl.h) and the small tile, twenty
+// FP64 steps took, us: 96 x 80 1005 -> 549, 200^2 1258 -> 857, 512^2 3185 ->
+// 2793; at 4096^2 7.24 -> 7.21 ms a step.
+__global__ void k_publish(const double* blk, const double* fixed, const double* alpha_cur, int cur, double* zero,
+                          double* host, unsigned long long seq)
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int k = threadIdx.x;
+    if (k < BLOCK) zero[k] = 0.0;
+    if (k < NSLOTS) {
+        double v = k < SLOT_SMAX_ALT ? blk[k] : fixed[k - SLOT_SMAX_ALT];
+        const int c = k - (SLOT_ALPHA + 2 * cur);
+        if (c == 0 || c == 1) v = alpha_cur[c];
+        *const_cast<volatile double*>(host + k) = v;
+    }
+    __threadfence_system();
+    __syncwarp();
+    if (k == 0) *reinterpret_cast<volatile unsigned long long*>(host + SLOT_SEQ) = seq;
 }
 
 // max |a - b| and max |b| over all planes' interior values (judge step).
@@ -355,8 +391,8 @@ int buffer_of(const fin_solver* s, const double* ptr)
     return -1;
 }
 
-template <class R, int VER, bool P2, bool FG = false>
-int launch_stage_t(fin_solver* s, const StageArgs& a)
+template <class R, int VER, bool P2, bool FG, class Cfg>
+int launch_stage_cfg(fin_solver* s, const StageArgs& a)
 {
     const size_t smem = Cfg::template smem_bytes<R>();
     auto kern = k_stage<R, VER, P2, Cfg, FG>;
@@ -366,10 +402,27 @@ int launch_stage_t(fin_solver* s, const StageArgs& a)
         configured = true;
     }
     dim3 grid((a.my + Cfg::TJ - 1) / Cfg::TJ, (a.mx + Cfg::TI - 1) / Cfg::TI);
-    kern<<<grid, Cfg::NT, smem, s->stream>>>(a);
+    CK(launch_pdl(kern, grid, dim3(Cfg::NT), smem, s->stream, a));
     s->launches++;
-    CK(cudaGetLastError());
     return FIN_OK;
+}
+
+// FP64 grids of at most SMALL tiles of 15 x 16 leave SMs idle or give some of
+// them twice the work of others: tiles of 7 x 16 with a thread for every face
+// (one round instead of two) spread them.  Twenty steps, us, 15 x 16 / 7 x 16
+// (before the launch work below): 64^2 980 / 872, 128^2 990 / 953, 160^2 1002 /
+// 1002, 200^2 (182 tiles) 1249 / 1206; from 256^2 (288) on the larger tile wins,
+// 1260 / 1443.
+constexpr int SMALL = 200;
+using SmallCfg = TileCfg<7, 16, 256>;
+
+template <class R, int VER, bool P2, bool FG = false>
+int launch_stage_t(fin_solver* s, const StageArgs& a)
+{
+    const long long tiles = (long long)((a.mx + Cfg::TI - 1) / Cfg::TI) * ((a.my + Cfg::TJ - 1) / Cfg::TJ);
+    if constexpr (sizeof(R) == 8)
+        if (tiles <= SMALL) return launch_stage_cfg<R, VER, P2, FG, SmallCfg>(s, a);
+    return launch_stage_cfg<R, VER, P2, FG, Cfg>(s, a);
 }
 
 template <class R>
@@ -421,9 +474,8 @@ int launch_stage_hyb_t(fin_solver* s, const StageArgs& a)
         if (ext) b.tm_A = s->tm_a[ie];
     }
     const long long tiles = (long long)((a.mx + HybCfg::TI - 1) / HybCfg::TI) * ((a.my + HybCfg::TJ - 1) / HybCfg::TJ);
-    kern<<<unsigned(tiles), HybCfg::NT, Lh::BYTES, s->stream>>>(b);
+    CK(launch_pdl(kern, dim3(unsigned(tiles)), dim3(HybCfg::NT), Lh::BYTES, s->stream, b));
     s->launches++;
-    CK(cudaGetLastError());
     return FIN_OK;
 }
 
@@ -527,12 +579,59 @@ int grid_blocks(size_t n)
     return int(b);
 }
 
-double* alpha_slot(fin_solver* s, int buf) { return s->slots + SLOT_ALPHA + 2 * buf; }
+double* alpha_slot(fin_solver* s, int buf) { return s->slots + BLOCK * s->ablk[buf] + SLOT_ALPHA + 2 * buf; }
+double* smax_slot(fin_solver* s) { return s->slots + BLOCK * s->cb + SLOT_SMAX; }
+
+// A step from q[cur] begins: its block becomes the one that is all zero, and
+// the buffers it may write keep their wave speeds there.
+int begin_step(fin_solver* s)
+{
+    int z = s->zb;
+    if (z < 0) {
+        z = (s->ablk[s->cur] + 1) % NBLOCK;
+        CK(cudaMemsetAsync(s->slots + BLOCK * z, 0, BLOCK * sizeof(double), s->stream));
+    }
+    s->zb = -1;
+    s->cb = z;
+    s->status = reinterpret_cast<unsigned int*>(s->slots + BLOCK * z + SLOT_STATUS);
+    for (int b = 0; b < NBUF; b++)
+        if (b != s->cur) s->ablk[b] = z;
+    return FIN_OK;
+}
+
+// The step's slots in the host's mirror (s->h_slots), when all its kernels
+// have finished.
+int finish_step(fin_solver* s)
+{
+    int z = 0;
+    while (z == s->cb || z == s->ablk[s->cur]) z++;
+    const unsigned long long seq = ++s->seq;
+    CK(launch_pdl(k_publish, dim3(1), dim3(32), 0, s->stream, (const double*)(s->slots + BLOCK * s->cb),
+                  (const double*)(s->slots + FIXED), (const double*)alpha_slot(s, s->cur), s->cur,
+                  s->slots + BLOCK * z, s->h_slots, seq));
+    s->launches++;
+    s->zb = z;
+    const volatile unsigned long long* got = reinterpret_cast<volatile unsigned long long*>(s->h_slots + SLOT_SEQ);
+    for (unsigned n = 1; *got != seq; n++) {
+        if (n % 65536 == 0) {   // the stream stopped without the number: its error, if the number still is not there
+            const cudaError_t e = cudaStreamQuery(s->stream);
+            if (e != cudaErrorNotReady && *got != seq) {
+                CK(e);
+                CK(cudaStreamSynchronize(s->stream));
+                if (*got != seq) return set_err(FIN_ERR_CUDA, "a step ended without its result");
+            }
+        }
+    }
+    std::atomic_thread_fence(std::memory_order_acquire);
+    if (s->time_kernels) CK(cudaStreamSynchronize(s->stream));   // the stages' events
+    return FIN_OK;
+}
 
 // Global alpha of buffer buf into its slot (used when no stage epilogue has
 // produced it: after set_state, or when global_alpha is off it is unused).
 int compute_alpha(fin_solver* s, int buf)
 {
+    if (buf != s->cur) s->ablk[buf] = s->cb;   // never the block that is all zero
     CK(cudaMemsetAsync(alpha_slot(s, buf), 0, 2 * sizeof(double), s->stream));
     const size_t n = size_t(s->p.mx) * s->p.my;
     k_wave_spd_max<<<grid_blocks(n), 256, 0, s->stream>>>(s->q[buf], s->p.mx, s->p.my, s->plane, s->p.gamma,
@@ -636,13 +735,10 @@ int take_stage_lxw_mpp(fin_solver* s, double dt, int nxt)
     if (!s->mpp_fx) CK(cudaMalloc(&s->mpp_fx, MEQN * nx * sizeof(double)));
     if (!s->mpp_fy) CK(cudaMalloc(&s->mpp_fy, MEQN * ny * sizeof(double)));
     if (!s->mpp_amin) CK(cudaMalloc(&s->mpp_amin, 4 * nc * sizeof(double)));
-    CK(cudaMemsetAsync(s->slots + SLOT_SMAX, 0, 2 * sizeof(double), s->stream));
-    CK(cudaMemsetAsync(s->slots + SLOT_STATUS, 0, sizeof(double), s->stream));
-    CK(cudaMemsetAsync(alpha_slot(s, nxt), 0, 2 * sizeof(double), s->stream));
     int rc;
     if ((rc = launch_intflux(s, p.time_order > 2 ? 1 : 0, s->q[qn], nullptr, dt, 0, 0, 0, 0))) return rc;
     StageArgs a = base_args(s);
-    a.smax_out = s->slots + SLOT_SMAX;
+    a.smax_out = smax_slot(s);
     a.Fg = s->Fg; a.Gg = s->Gg; a.gplane = s->gplane;
     a.qin = s->q[qn]; a.A = s->q[qn]; a.B = nullptr; a.qout = s->q[nxt];
     a.a1 = 1.0; a.a2 = 0.0; a.bdt = dt;
@@ -686,14 +782,10 @@ int take_stages_lw(fin_solver* s, double dt, int nxt)
     const int qn = s->cur;
     int q1 = 0;
     while (q1 == qn || q1 == nxt) q1++;
-    CK(cudaMemsetAsync(s->slots + SLOT_SMAX, 0, 2 * sizeof(double), s->stream));
-    CK(cudaMemsetAsync(s->slots + SLOT_STATUS, 0, sizeof(double), s->stream));
-    CK(cudaMemsetAsync(alpha_slot(s, q1), 0, 2 * sizeof(double), s->stream));
-    CK(cudaMemsetAsync(alpha_slot(s, nxt), 0, 2 * sizeof(double), s->stream));
     const bool ga = p.global_alpha != 0;
     int rc;
     StageArgs a = base_args(s);
-    a.smax_out = s->slots + SLOT_SMAX;
+    a.smax_out = smax_slot(s);
     a.Fg = s->Fg; a.Gg = s->Gg; a.gplane = s->gplane;
     if (p.time_stepping_method == FIN_TS_LXW && p.mpp_limiter) return take_stage_lxw_mpp(s, dt, nxt);
     if (p.time_stepping_method == FIN_TS_LXW) {
@@ -762,8 +854,9 @@ void stage_registers(fin_solver* s, int nxt, int* q1, int* q2)
 int take_stages(fin_solver* s, double dt, int nxt)
 {
     s->judge_pending = false;
-    if (s->p.time_stepping_method != FIN_TS_RK) return take_stages_lw(s, dt, nxt);
     int q1, q2, rc;
+    if ((rc = begin_step(s))) return rc;
+    if (s->p.time_stepping_method != FIN_TS_RK) return take_stages_lw(s, dt, nxt);
     stage_registers(s, nxt, &q1, &q2);
     if (s->p.precision != FIN_PREC_HYBRID || !s->mlpP) return take_stages_rk(s, dt, nxt, nullptr, q1, q2);
     // Hybrid form: flags from the indicator on q^n, FP32 stages with the
@@ -786,16 +879,21 @@ int take_stages(fin_solver* s, double dt, int nxt)
     if ((rc = take_stages_rk(s, dt, nxt, s->flags, q1, q2))) return rc;
     s->hstep++;
     if (s->judge_every > 0 && s->hstep % s->judge_every == 0) {
-        CK(cudaMemcpyAsync(s->slots + SLOT_SMAX_ALT, s->slots + SLOT_SMAX, 2 * sizeof(double), cudaMemcpyDeviceToDevice,
-                           s->stream));
+        // the judge's stages use the step's block again: its maxima move to
+        // SMAX_ALT (the host's mirror), everything it adds into is zeroed
+        CK(cudaMemcpyAsync(s->slots + FIXED, smax_slot(s), 2 * sizeof(double), cudaMemcpyDeviceToDevice, s->stream));
+        CK(cudaMemsetAsync(smax_slot(s), 0, 2 * sizeof(double), s->stream));
+        CK(cudaMemsetAsync(s->status, 0, sizeof(double), s->stream));
+        CK(cudaMemsetAsync(alpha_slot(s, q1), 0, 2 * sizeof(double), s->stream));
+        CK(cudaMemsetAsync(alpha_slot(s, q2), 0, 2 * sizeof(double), s->stream));
         const bool tk = s->time_kernels;   // the step's stage times stay those of the hybrid stages
         s->time_kernels = false;
         rc = take_stages_rk(s, dt, 4, nullptr, q1, q2);
         s->time_kernels = tk;
         if (rc) return rc;
-        CK(cudaMemsetAsync(s->slots + SLOT_DIFF, 0, 2 * sizeof(double), s->stream));
+        CK(cudaMemsetAsync(s->slots + FIXED + 2, 0, 2 * sizeof(double), s->stream));
         const size_t n = size_t(s->p.mx) * s->p.my;
-        k_max_diff<<<grid_blocks(n), 256, 0, s->stream>>>(s->q[nxt], s->q[4], s->plane, n, s->slots + SLOT_DIFF);
+        k_max_diff<<<grid_blocks(n), 256, 0, s->stream>>>(s->q[nxt], s->q[4], s->plane, n, s->slots + FIXED + 2);
         s->launches++;
         CK(cudaGetLastError());
         s->judge_pending = true;
@@ -854,11 +952,9 @@ int take_stages_rk_other(fin_solver* s, double dt, int nxt)
     const int qn = s->cur;
     int r1, r2;
     stage_registers(s, nxt, &r1, &r2);
-    CK(cudaMemsetAsync(s->slots + SLOT_SMAX, 0, 2 * sizeof(double), s->stream));
-    CK(cudaMemsetAsync(s->slots + SLOT_STATUS, 0, sizeof(double), s->stream));
     const bool ga = p.global_alpha != 0;
     StageArgs a = base_args(s);
-    a.smax_out = s->slots + SLOT_SMAX;
+    a.smax_out = smax_slot(s);
     int k = 0;
     // q[out] = a1 q[A] + a2 q[B] + bdt L(q[in]); A, B < 0: term absent
     auto stage = [&](int in, int A, double a1, int B, double a2, double bdt, int out) -> int {
@@ -932,17 +1028,10 @@ int take_stages_rk(fin_solver* s, double dt, int nxt, const unsigned* flags, int
     const fin_params& p = s->p;
     if (p.time_order != 3) return take_stages_rk_other(s, dt, nxt);
     const int qn = s->cur;
-    // reset smax, the status word and the alpha slots of the three buffers
-    // written this step
-    CK(cudaMemsetAsync(s->slots + SLOT_SMAX, 0, 2 * sizeof(double), s->stream));
-    CK(cudaMemsetAsync(s->slots + SLOT_STATUS, 0, sizeof(double), s->stream));
-    CK(cudaMemsetAsync(alpha_slot(s, q1), 0, 2 * sizeof(double), s->stream));
-    CK(cudaMemsetAsync(alpha_slot(s, q2), 0, 2 * sizeof(double), s->stream));
-    CK(cudaMemsetAsync(alpha_slot(s, nxt), 0, 2 * sizeof(double), s->stream));
     const bool ga = p.global_alpha != 0;
     int rc;
     StageArgs a = base_args(s);
-    a.smax_out = s->slots + SLOT_SMAX;
+    a.smax_out = smax_slot(s);
     a.flags = flags;
     // stage 1: q1 = 1*q^n + 0*q* + (1*dt) L(q^n)
     a.qin = s->q[qn]; a.A = s->q[qn]; a.B = nullptr; a.qout = s->q[q1];
@@ -973,8 +1062,8 @@ int take_stages_rk(fin_solver* s, double dt, int nxt, const unsigned* flags, int
 // simply retried); the caller refuses to accept it.
 int get_cfl(fin_solver* s, double dt, double dtmax, double* cfl, bool* nonfinite)
 {
-    CK(cudaMemcpyAsync(s->h_slots, s->slots, NSLOTS * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
-    CK(cudaStreamSynchronize(s->stream));
+    const int rf = finish_step(s);
+    if (rf) return rf;
     unsigned int st;
     memcpy(&st, s->h_slots + SLOT_STATUS, sizeof(st));
     *nonfinite = (st & 1u) != 0;
@@ -1138,9 +1227,11 @@ int fin_create(const fin_params* p, fin_solver** out)
         if ((e = cudaMalloc(&s->Fg, MEQN * s->gplane * sizeof(double))) != cudaSuccess) return fail(e, "cudaMalloc F");
         if ((e = cudaMalloc(&s->Gg, MEQN * s->gplane * sizeof(double))) != cudaSuccess) return fail(e, "cudaMalloc G");
     }
-    if ((e = cudaMalloc(&s->slots, NSLOTS * sizeof(double))) != cudaSuccess) return fail(e, "cudaMalloc slots");
-    s->status = reinterpret_cast<unsigned int*>(s->slots + SLOT_STATUS);
-    if ((e = cudaMallocHost(&s->h_slots, NSLOTS * sizeof(double))) != cudaSuccess) return fail(e, "cudaMallocHost");
+    if ((e = cudaMalloc(&s->slots, NDEV * sizeof(double))) != cudaSuccess) return fail(e, "cudaMalloc slots");
+    s->status = reinterpret_cast<unsigned int*>(s->slots + SLOT_STATUS);   // block 0 (cb), all buffers' wave speeds there
+    s->zb = 1;
+    if ((e = cudaMallocHost(&s->h_slots, (NSLOTS + 1) * sizeof(double))) != cudaSuccess) return fail(e, "cudaMallocHost");
+    memset(s->h_slots, 0, (NSLOTS + 1) * sizeof(double));
     if ((e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking)) != cudaSuccess) return fail(e, "stream");
     if ((e = cudaEventCreate(&s->ev0)) != cudaSuccess) return fail(e, "event");
     if ((e = cudaEventCreate(&s->ev1)) != cudaSuccess) return fail(e, "event");
@@ -1148,7 +1239,7 @@ int fin_create(const fin_params* p, fin_solver** out)
         if ((e = cudaEventCreate(&s->kev[k])) != cudaSuccess) return fail(e, "event");
     for (int k = 0; k < 2; k++)
         if ((e = cudaEventCreate(&s->iev[k])) != cudaSuccess) return fail(e, "event");
-    if ((e = cudaMemsetAsync(s->slots, 0, NSLOTS * sizeof(double), s->stream)) != cudaSuccess) return fail(e, "memset");
+    if ((e = cudaMemsetAsync(s->slots, 0, NDEV * sizeof(double), s->stream)) != cudaSuccess) return fail(e, "memset");
     for (int b = 0; b < nbuf; b++)
         if ((e = cudaMemsetAsync(s->q[b], 0, MEQN * s->plane * sizeof(double), s->stream)) != cudaSuccess) return fail(e, "memset");
     if ((e = cudaStreamSynchronize(s->stream)) != cudaSuccess) return fail(e, "sync");
@@ -1202,7 +1293,7 @@ static int upload(fin_solver* s, const double* q_host, int buf)
 {
     int rc = ensure_aos(s);
     if (rc) return rc;
-    CK(cudaMemsetAsync(s->slots + SLOT_STATUS, 0, sizeof(double), s->stream));
+    CK(cudaMemsetAsync(s->status, 0, sizeof(double), s->stream));
     CK(cudaMemcpyAsync(s->d_aos, q_host, s->aos_elems * sizeof(double), cudaMemcpyHostToDevice, s->stream));
     const size_t n = size_t(s->p.mx) * s->p.my;
     k_aos_to_planes<<<grid_blocks(n), 256, 0, s->stream>>>(s->d_aos, s->q[buf], s->p.mx, s->p.my, s->p.mbc, s->plane);
@@ -1218,7 +1309,7 @@ int fin_set_state(fin_solver* s, const double* q_host, double t)
     if (rc) return rc;
     s->t = t;
     s->ind_since = -1;
-    CK(cudaMemsetAsync(s->slots + SLOT_STATUS, 0, sizeof(double), s->stream));
+    CK(cudaMemsetAsync(s->status, 0, sizeof(double), s->stream));
     if ((rc = compute_alpha(s, s->cur))) return rc;
     s->alpha_valid = true;
     return check_status(s);
@@ -1272,7 +1363,7 @@ int fin_set_state_qinit(fin_solver* s, int problem, const double* prm, int nprm,
     s->launches++;
     s->t = t;
     s->ind_since = -1;
-    CK(cudaMemsetAsync(s->slots + SLOT_STATUS, 0, sizeof(double), s->stream));
+    CK(cudaMemsetAsync(s->status, 0, sizeof(double), s->stream));
     int rc = compute_alpha(s, s->cur);
     if (rc) return rc;
     s->alpha_valid = true;
@@ -1676,13 +1767,13 @@ int fin_get_cfl(fin_solver* s, double dt, double dtmax, const double* smax_host,
     if (rc) return rc;
     if (n > s->aos_elems) return set_err(FIN_ERR_ARG, "smax larger than the staging buffer");
     CK(cudaMemcpyAsync(s->d_aos, smax_host, n * sizeof(double), cudaMemcpyHostToDevice, s->stream));
-    CK(cudaMemsetAsync(s->slots + SLOT_SMAX_ALT, 0, 2 * sizeof(double), s->stream));
+    CK(cudaMemsetAsync(s->slots + FIXED, 0, 2 * sizeof(double), s->stream));
     const size_t cells = size_t(p.mx) * p.my;
-    k_smax_max<<<grid_blocks(cells), 256, 0, s->stream>>>(s->d_aos, p.mx, p.my, p.mbc, s->slots + SLOT_SMAX_ALT);
+    k_smax_max<<<grid_blocks(cells), 256, 0, s->stream>>>(s->d_aos, p.mx, p.my, p.mbc, s->slots + FIXED);
     s->launches++;
     CK(cudaGetLastError());
     double h[2];
-    CK(cudaMemcpyAsync(h, s->slots + SLOT_SMAX_ALT, sizeof(h), cudaMemcpyDeviceToHost, s->stream));
+    CK(cudaMemcpyAsync(h, s->slots + FIXED, sizeof(h), cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
     double c = -100.0;
     c = Max(dt * h[0] / s->dx, c);
@@ -1724,6 +1815,7 @@ int fin_step_fixed(fin_solver* s, double dt, double* cfl_out)
     settle_judge(s, nxt, dt, &cfl);
     if (nonfinite) return set_err(FIN_ERR_NONFINITE, "non-finite wave speed or state");
     float ms = 0.f;
+    CK(cudaEventSynchronize(s->ev1));
     CK(cudaEventElapsedTime(&ms, s->ev0, s->ev1));
     s->last_ms = ms;
     s->cur = nxt;
@@ -2031,7 +2123,7 @@ int fin_read_frame(fin_solver* s, const char* path)
     s->launches++;
     s->t = t;
     s->ind_since = -1;
-    CK(cudaMemsetAsync(s->slots + SLOT_STATUS, 0, sizeof(double), s->stream));
+    CK(cudaMemsetAsync(s->status, 0, sizeof(double), s->stream));
     int r2 = compute_alpha(s, s->cur);
     if (r2) return r2;
     s->alpha_valid = true;

@@ -5,15 +5,16 @@ reconstruction form and with both kinds of boundaries, against the oracle.
 Tolerance: the plain form's 1e-12 relative L-infinity.  A right-hand side
 divides flux differences by dx, so a relative rounding error u = 1.1e-16 of the
 fluxes (some tens of operations deep, fluxes of order 3 here) reaches L as
-about 50 u |F| / (dx |L|); on these grids |L| >= 1 and 1/dx <= 64, hence below
-1.1e-12 in the worst case and far below it in practice.
+about 50 u |F| / (dx |L|); on the small grids |L| >= 1 and 1/dx <= 64, hence
+below 1.1e-12 in the worst case and far below it in practice (rounding errors
+do not align), which leaves room for the finer grids of the tile rule.
 """
 import numpy as np
 import pytest
 
 from conftest import interior, rel_linf
 from finess_b200 import problems as P
-from finess_b200._abi import FIN_WENO_FD, FIN_WENO_JS, FIN_WENO_Z
+from finess_b200._abi import FIN_TS_LXW, FIN_TS_MD, FIN_WENO_FD, FIN_WENO_JS, FIN_WENO_Z
 
 pytestmark = pytest.mark.gpu
 
@@ -36,6 +37,38 @@ def _problem(mx, my, periodic, weno, power, local, rng):
 @pytest.mark.parametrize("mx,my,periodic", [(1, 1, False), (1, 40, False), (14, 15, False), (15, 16, True), (16, 17, True),
                                             (3, 64, True), (31, 33, False), (61, 50, True)])
 def test_construct_l_and_step_at_tile_edges(oracle, mx, my, periodic, weno, power):
+    _check(oracle, mx, my, periodic, weno, power)
+
+
+# The count of 15 x 16 tiles at which FP64 stages turn from 7 x 16 to 15 x 16
+# tiles is 200: grids of 240, 272, 224 (15 x 16 tiles) and of 200, 195 tiles.
+@pytest.mark.parametrize("weno,power", [(FIN_WENO_JS, 2.0), (FIN_WENO_Z, 2.0), (FIN_WENO_FD, 2.0), (FIN_WENO_Z, 1.5)])
+@pytest.mark.parametrize("mx,my,periodic", [(240, 240, True), (241, 257, False), (209, 255, True), (150, 320, False),
+                                            (195, 240, True)])
+def test_either_side_of_the_tile_rule(oracle, mx, my, periodic, weno, power):
+    _check(oracle, mx, my, periodic, weno, power)
+
+
+@pytest.mark.parametrize("method,time_order", [(FIN_TS_MD, 4), (FIN_TS_LXW, 3)])
+@pytest.mark.parametrize("mx,my", [(241, 225), (64, 49)])
+def test_integrated_flux_steps_on_either_tile(oracle, mx, my, method, time_order):
+    """Two steps of the multiderivative and Lax-Wendroff methods (1e-11: the
+    bar of whole frames)."""
+    from finess_b200.solver import Solver
+    rng = np.random.default_rng(mx)
+    p = P.riemann_params(n=mx, weno=FIN_WENO_Z, mbc=5, time_stepping_method=method, time_order=time_order)
+    p.my, p.yhigh = my, my / mx
+    q = oracle.set_bnd(p, P.random_smooth_state(p, rng))
+    dt = p.max_dt = 0.05 / mx
+    with Solver(p) as s:
+        s.set_state(q)
+        s.FinSolveRK(2 * dt, [0.0, dt, dt])
+        q1, _ = s.get_state()
+    qo = oracle.finsolve(p, q, 0.0, 2 * dt, dt)[1]
+    assert rel_linf(interior(p, q1), interior(p, qo)) <= 1e-11
+
+
+def _check(oracle, mx, my, periodic, weno, power):
     from finess_b200.solver import Solver
     rng = np.random.default_rng(100 * mx + my)
     p, q = _problem(mx, my, periodic, weno, power, mx % 2 == 0, rng)
