@@ -23,6 +23,7 @@
 #include "fin_hybrid.cuh"
 #include "fin_tmap.h"
 #include "fin_pdl.h"
+#include "fin_hostio.h"
 #include "fin_output.h"
 #include "fin_mpp.cuh"
 #include "fin_rk.cuh"
@@ -89,6 +90,7 @@ struct fin_solver {
     int ablk[NBUF];         // block that holds the global wave speeds of each buffer
     unsigned long long seq; // steps published
     double* d_aos;          // staging buffer for the reference ghosted layout
+    HostRing ring;          // pinned chunks on the way to L and smax
     size_t aos_elems;
     double* d_aux;          // second staging / L output buffer (planes)
     double* Fg;             // integrated fluxes F, G (Lax-Wendroff / multiderivative)
@@ -345,16 +347,24 @@ __global__ void k_planes_to_aos(const double* planes, double* aos, int mx, int m
     }
 }
 
-// Interior planes -> interior of a ghosted AoS array, ghosts untouched.
-__global__ void k_planes_to_aos_interior(const double* planes, double* aos, int mx, int my, int mbc, size_t plane)
+// Interior planes -> packed cells (i, j, m), m fastest.
+__global__ void k_planes_to_cells(const double* planes, double* cells, size_t n, size_t plane)
 {
-    const size_t n = size_t(mx) * my;
-    const int sy = my + 2 * mbc;
+    for (size_t e = blockIdx.x * size_t(blockDim.x) + threadIdx.x; e < n * MEQN; e += size_t(gridDim.x) * blockDim.x) {
+        const size_t g = e / MEQN;
+        cells[e] = planes[(e - g * MEQN) * plane + g];
+    }
+}
+
+// Face speeds of both directions -> (i, j, 2), i = 0..mx, j = 0..my; the x
+// face (i, my) and the y face (mx, j) do not exist.
+__global__ void k_faces_to_smax(const double* fx, const double* fy, double* sm, int mx, int my)
+{
+    const size_t w = size_t(my) + 1, n = (size_t(mx) + 1) * w;
     for (size_t g = blockIdx.x * size_t(blockDim.x) + threadIdx.x; g < n; g += size_t(gridDim.x) * blockDim.x) {
-        const int i = int(g / my), j = int(g - size_t(i) * my);
-        const size_t dst = (size_t(i + mbc) * sy + (j + mbc)) * MEQN;
-#pragma unroll
-        for (int m = 0; m < MEQN; m++) aos[dst + m] = planes[m * plane + g];
+        const size_t i = g / w, j = g - i * w;
+        sm[2 * g] = j < size_t(my) ? fx[i * my + j] : 0.0;
+        sm[2 * g + 1] = i < size_t(mx) ? fy[i * w + j] : 0.0;
     }
 }
 
@@ -410,7 +420,7 @@ int launch_stage_cfg(fin_solver* s, const StageArgs& a)
 // FP64 grids of at most SMALL tiles of 15 x 16 leave SMs idle or give some of
 // them twice the work of others: tiles of 7 x 16 with a thread for every face
 // (one round instead of two) spread them.  Twenty steps, us, 15 x 16 / 7 x 16
-// (before the launch work below): 64^2 980 / 872, 128^2 990 / 953, 160^2 1002 /
+// (with five memsets and a copy a step): 64^2 980 / 872, 128^2 990 / 953, 160^2 1002 /
 // 1002, 200^2 (182 tiles) 1249 / 1206; from 256^2 (288) on the larger tile wins,
 // 1260 / 1443.
 constexpr int SMALL = 200;
@@ -1265,6 +1275,7 @@ int fin_destroy(fin_solver* s)
     cudaFree(s->ind_count);
     cudaFree(s->slots);
     cudaFree(s->d_aos);
+    s->ring.destroy();
     cudaFree(s->d_aux);
     cudaFree(s->Fg);
     cudaFree(s->Gg);
@@ -1403,7 +1414,7 @@ int fin_global_wave_spd(fin_solver* s, const double* q_host, double* alpha1, dou
     return check_status(s);
 }
 
-static int download_l_smax(fin_solver* s, int outb, double* L_host, double* smax_host);
+static int download_l_smax(fin_solver* s, int buf, int outb, double* L_host, double* smax_host);
 
 int fin_construct_l(fin_solver* s, const double* q_host, double* L_host, double* smax_host)
 {
@@ -1425,50 +1436,53 @@ int fin_construct_l(fin_solver* s, const double* q_host, double* L_host, double*
     a.face_alpha_x = smax_host ? s->d_face_x : nullptr;
     a.face_alpha_y = smax_host ? s->d_face_y : nullptr;
     if ((rc = launch_stage(s, a))) return rc;
-    return download_l_smax(s, outb, L_host, smax_host);
+    return download_l_smax(s, buf, outb, L_host, smax_host);
 }
 
 // L (interior of the ghosted output, ghosts untouched: the reference leaves
 // Lstar's ghost entries uninitialised) from q[outb], and smax max-accumulated
-// from the per-face speeds, then the status word.
-static int download_l_smax(fin_solver* s, int outb, double* L_host, double* smax_host)
+// from the per-face speeds, then the status word.  Both are laid out on the
+// device, so the host moves whole rows: L's packed cells go to q[buf] (the input
+// state, read by now, of the same size), smax to the staging buffer.  300 x 257
+// with both: 1650 -> 755 us, 1000 x 1100: 35 -> 11.4 ms (planes copied into a
+// zeroed vector and transposed by the host before).
+static int download_l_smax(fin_solver* s, int buf, int outb, double* L_host, double* smax_host)
 {
     const fin_params& p = s->p;
-    const size_t n = size_t(p.mx) * p.my;
-    std::vector<double> hl(MEQN * n);
-    for (int m = 0; m < MEQN; m++)
-        CK(cudaMemcpyAsync(hl.data() + m * n, s->q[outb] + m * s->plane, n * sizeof(double), cudaMemcpyDeviceToHost,
-                           s->stream));
-    CK(cudaStreamSynchronize(s->stream));
-    {
-        const int sy = p.my + 2 * p.mbc;
-        for (int i = 0; i < p.mx; i++)
-            for (int j = 0; j < p.my; j++)
-                for (int m = 0; m < MEQN; m++)
-                    L_host[(size_t(i + p.mbc) * sy + (j + p.mbc)) * MEQN + m] = hl[m * n + size_t(i) * p.my + j];
-    }
+    const size_t n = size_t(p.mx) * p.my, ns = 2 * (size_t(p.mx) + 1) * (size_t(p.my) + 1);
+    k_planes_to_cells<<<grid_blocks(MEQN * n), 256, 0, s->stream>>>(s->q[outb], s->q[buf], n, s->plane);
+    s->launches++;
+    CK(cudaGetLastError());
     if (smax_host) {
-        std::vector<double> fx(size_t(p.mx + 1) * p.my), fy(size_t(p.mx) * (p.my + 1));
-        CK(cudaMemcpyAsync(fx.data(), s->d_face_x, fx.size() * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
-        CK(cudaMemcpyAsync(fy.data(), s->d_face_y, fy.size() * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
-        CK(cudaStreamSynchronize(s->stream));
-        // smax is dTensorBC3(mx+1, my+1, 2, mbc): max-accumulate (ConstructL.cpp:173,324)
-        const int sy = p.my + 1 + 2 * p.mbc;
-        auto at = [&](int i, int j, int m) -> double& {   // 1-based i, j, m
-            return smax_host[(size_t(i + p.mbc - 1) * sy + (j + p.mbc - 1)) * 2 + (m - 1)];
-        };
-        for (int i = 1; i <= p.mx + 1; i++)
-            for (int j = 1; j <= p.my; j++) {
-                double& d = at(i, j, 1);
-                d = Max(d, fx[size_t(i - 1) * p.my + (j - 1)]);
-            }
-        for (int i = 1; i <= p.mx; i++)
-            for (int j = 1; j <= p.my + 1; j++) {
-                double& d = at(i, j, 2);
-                d = Max(d, fy[size_t(i - 1) * (p.my + 1) + (j - 1)]);
-            }
+        k_faces_to_smax<<<grid_blocks(ns / 2), 256, 0, s->stream>>>(s->d_face_x, s->d_face_y, s->d_aos, p.mx, p.my);
+        s->launches++;
+        CK(cudaGetLastError());
     }
-    CK(cudaStreamSynchronize(s->stream));
+    const size_t row = size_t(p.my) * MEQN, ldl = size_t(p.my + 2 * p.mbc) * MEQN;
+    CK(s->ring.down(s->q[buf], MEQN * n, s->stream, [&](size_t o, const double* c, size_t len) {
+        for (size_t i = o / row, k = o - i * row, m; len > 0; i++, k = 0, c += m, len -= m) {
+            m = row - k < len ? row - k : len;
+            memcpy(L_host + (i + p.mbc) * ldl + p.mbc * MEQN + k, c, m * sizeof(double));
+        }
+    }));
+    if (smax_host) {
+        // smax is dTensorBC3(mx+1, my+1, 2, mbc): max-accumulate (ConstructL.cpp:173,324)
+        const size_t rs = 2 * (size_t(p.my) + 1), lds = 2 * size_t(p.my + 1 + 2 * p.mbc);
+        CK(s->ring.down(s->d_aos, ns, s->stream, [&](size_t o, const double* c, size_t len) {
+            for (size_t i = o / rs, k = o - i * rs, m; len > 0; i++, k = 0, c += m, len -= m) {
+                m = rs - k < len ? rs - k : len;
+                double* d = smax_host + (i + p.mbc) * lds + 2 * p.mbc + k;
+                if (i == size_t(p.mx)) {   // x faces only
+                    for (size_t e = k & 1; e < m; e += 2)
+                        if (k + e < rs - 2) d[e] = Max(d[e], c[e]);
+                    continue;
+                }
+                const size_t stop = m < rs - 2 - k || k > rs - 2 ? m : rs - 2 - k;   // before the missing x face
+                for (size_t e = 0; e < stop; e++) d[e] = Max(d[e], c[e]);
+                if (k <= rs - 2 && k + m > rs - 1) d[rs - 1 - k] = Max(d[rs - 1 - k], c[rs - 1 - k]);
+            }
+        }));
+    }
     return check_status(s);
 }
 
@@ -1699,7 +1713,7 @@ int fin_construct_lxwl(fin_solver* s, const double* q_host, const double* F_host
                             fy[(size_t(m) * p.mx + i) * (p.my + 1) + j];
         }
     }
-    return download_l_smax(s, outb, L_host, smax_host);
+    return download_l_smax(s, buf, outb, L_host, smax_host);
 }
 
 // UpdateSoln (lib/2d/UpdateSoln.cpp:14-38) on ghosted host arrays: every
