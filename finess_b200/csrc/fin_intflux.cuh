@@ -23,11 +23,20 @@
 //
 // One block computes a TI x TJ tile of output cells; q is staged with a
 // 2-cell halo (boundary conditions by remap), f and g are evaluated once per
-// staged cell, then one thread per output cell forms F and G.  Output arrays
-// are ghosted planes of (mx+6) x (my+6): cell (i, j), i in [-3, mx+3), sits at
-// (i+3)*(my+6) + (j+3).
+// staged cell, then one thread per output cell forms F and G.  The shared-memory
+// pipe and the FP64 pipe bound it, so a plane is staged once: f's density
+// component is q's x momentum, g's the y momentum, and both fluxes share
+// rho u v (15 planes -> 12; 9 without f_tt, whose centre cell's density, z
+// momentum and energy come from L2), and the differences' factors and the grid
+// spacings are one constant.  A block loads, then computes, so many small
+// blocks overlap better than few large ones: 8 x 16 against 16 x 16, with the
+// above, took two multiderivative steps at 1024 x 1000 from 1064 to 1039 us and
+// two Lax-Wendroff steps at 1023 x 1025 from 864 to 836 (8 x 32: 1055 / 857,
+// 4 x 32: 1042 / 854, 8 x 8: 1124 / 890).
+// Output arrays are ghosted planes of (mx+6) x (my+6): cell (i, j), i in
+// [-3, mx+3), sits at (i+3)*(my+6) + (j+3).
 #pragma once
-#include "fin_device.cuh"
+#include "fin_stage.cuh"
 
 namespace fin {
 
@@ -104,37 +113,49 @@ __device__ __forceinline__ void dflux2(double gamma, int n, const DCell& c, cons
              (c.E + c.p) * d2u[n - 1];
 }
 
-__device__ __forceinline__ double diff1(double rdx, double f0, double f1, double f3, double f4)
+// Diff1 and Diff2 with the factors of the stencil and of the grid in one:
+// k0 = 1 / 12 h, k1 = 2 / 3 h; l0 = -1 / 12 h^2, l1 = 4 / 3 h^2, l2 = -5 / 2 h^2.
+__device__ __forceinline__ double diff1(double k0, double k1, double f0, double f1, double f3, double f4)
 {
-    double tmp = (f0 - f4) * (1.0 / 12.0);
-    tmp += (-f1 + f3) * (2.0 / 3.0);
-    return tmp * rdx;
+    return fma(k0, f0 - f4, k1 * (f3 - f1));
 }
-__device__ __forceinline__ double diff2(double rdx2, double f0, double f1, double f2, double f3, double f4)
+__device__ __forceinline__ double diff2(double l0, double l1, double l2, double f0, double f1, double f2, double f3,
+                                        double f4)
 {
-    double tmp = (-f0 - f4) * (1.0 / 12.0);
-    tmp += (f1 + f3) * (4.0 / 3.0);
-    tmp += (-f2) * (5.0 / 2.0);
-    return tmp * rdx2;
+    return fma(l0, f0 + f4, fma(l1, f1 + f3, l2 * f2));
 }
 
 // MODE 0: 1-state, f_t only (time_order <= 2); 1: 1-state with f_tt; 2: 2-state;
 // 3: 2-state with f_tt (q2 null: the second state's terms, all with zero
 // coefficients, add nothing).
+template <int MODE>
+struct IntFluxPlanes {
+    static constexpr bool TT = MODE == 1 || MODE == 3;   // with f_tt: q's differences are wanted too
+    static constexpr int N = TT ? 12 : 9;
+    static constexpr int CTAS = MODE == 3 ? 4 : TT ? 5 : 6;   // of 128 threads: registers without much spilling
+    // TT: q0..q4, f1..f4, g2..g4; otherwise f0..f4, g0, g2..g4
+    static constexpr __host__ __device__ int f(int m) { return TT ? (m == 0 ? 1 : 4 + m) : m; }
+    static constexpr __host__ __device__ int g(int m)
+    {
+        return TT ? (m == 0 ? 2 : m == 1 ? 6 : 7 + m) : (m == 0 ? 5 : m == 1 ? 2 : 4 + m);
+    }
+};
+
 template <int MODE, int TI, int TJ>
-__global__ void __launch_bounds__(TI * TJ) k_intflux(const IntFluxArgs a)
+__global__ void __launch_bounds__(TI * TJ, IntFluxPlanes<MODE>::CTAS) k_intflux(const IntFluxArgs a)
 {
+    using P = IntFluxPlanes<MODE>;
     constexpr int HB = 2, BI = TI + 2 * HB, BJ = TJ + 2 * HB, PB = BI * BJ;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    double* qb = reinterpret_cast<double*>(smem_raw);   // [5][BI][BJ]
-    double* fb = qb + MEQN * PB;                       // [5][BI][BJ]  f
-    double* gb = fb + MEQN * PB;                       // [5][BI][BJ]  g
+    double* sb = reinterpret_cast<double*>(smem_raw);   // [P::N][BI][BJ]
+    grid_dependency();
     const int tid = threadIdx.x;
     const int i0 = int(blockIdx.y) * TI - 3, j0 = int(blockIdx.x) * TJ - 3;   // extended-domain origin
     const int ci = tid / TJ, cj = tid - ci * TJ;
     const int i = i0 + ci, j = j0 + cj;                // this thread's output cell
     const bool out_ok = i < a.mx + 3 && j < a.my + 3;
     const double rdx = 1.0 / a.dx, rdy = 1.0 / a.dy;
+    const double kx0 = rdx * (1.0 / 12.0), kx1 = rdx * (2.0 / 3.0), ky0 = rdy * (1.0 / 12.0), ky1 = rdy * (2.0 / 3.0);
     double Fo[MEQN] = {0, 0, 0, 0, 0}, Go[MEQN] = {0, 0, 0, 0, 0};
 
     const int nstate = (MODE == 2 || (MODE == 3 && a.q2)) ? 2 : 1;
@@ -157,6 +178,13 @@ __global__ void __launch_bounds__(TI * TJ) k_intflux(const IntFluxArgs a)
                 for (int m = 0; m < MEQN; m++) Qv[it][m] = __ldg(q + m * a.plane + g);
             }
         }
+        double Q[MEQN];
+        if (!P::TT) {
+            const size_t g = size_t(bc_remap(i, a.mx, a.bc[0], a.bc[1])) * a.my + bc_remap(j, a.my, a.bc[2], a.bc[3]);
+            Q[0] = __ldg(q + g);
+            Q[3] = __ldg(q + 3 * a.plane + g);
+            Q[4] = __ldg(q + 4 * a.plane + g);
+        }
 #pragma unroll
         for (int it = 0; it < NIT; it++) {
             const int e = tid + it * TI * TJ;
@@ -165,25 +193,33 @@ __global__ void __launch_bounds__(TI * TJ) k_intflux(const IntFluxArgs a)
                 Euler::flux(a.gamma, Qv[it], f, gg);
 #pragma unroll
                 for (int m = 0; m < MEQN; m++) {
-                    qb[m * PB + e] = Qv[it][m];
-                    fb[m * PB + e] = f[m];
-                    gb[m * PB + e] = gg[m];
+                    if (P::TT) sb[m * PB + e] = Qv[it][m];
+                    if (!P::TT || m > 0) sb[P::f(m) * PB + e] = f[m];
+                    if (m > 1 || (!P::TT && m == 0)) sb[P::g(m) * PB + e] = gg[m];
                 }
             }
         }
         __syncthreads();
         const int c0 = (ci + HB) * BJ + (cj + HB);
-#define AT(arr, m, di, dj) arr[(m) * PB + c0 + (di) * BJ + (dj)]
-        double Q[MEQN], w[MEQN], qx[MEQN], qy[MEQN];
+#define QT(m, di, dj) sb[(m) * PB + c0 + (di) * BJ + (dj)]
+#define FT(m, di, dj) QT(P::f(m), di, dj)
+#define GT(m, di, dj) QT(P::g(m), di, dj)
+        if (P::TT) {
+#pragma unroll
+            for (int m = 0; m < MEQN; m++) Q[m] = QT(m, 0, 0);
+        } else {
+            Q[1] = FT(0, 0, 0);
+            Q[2] = GT(0, 0, 0);
+        }
+        double w[MEQN], qx[MEQN], qy[MEQN];
 #pragma unroll
         for (int m = 0; m < MEQN; m++) {
-            Q[m] = AT(qb, m, 0, 0);
-            const double fx = diff1(rdx, AT(fb, m, -2, 0), AT(fb, m, -1, 0), AT(fb, m, 1, 0), AT(fb, m, 2, 0));
-            const double gy = diff1(rdy, AT(gb, m, 0, -2), AT(gb, m, 0, -1), AT(gb, m, 0, 1), AT(gb, m, 0, 2));
+            const double fx = diff1(kx0, kx1, FT(m, -2, 0), FT(m, -1, 0), FT(m, 1, 0), FT(m, 2, 0));
+            const double gy = diff1(ky0, ky1, GT(m, 0, -2), GT(m, 0, -1), GT(m, 0, 1), GT(m, 0, 2));
             w[m] = fx + gy;
-            if (MODE == 1 || MODE == 3) {
-                qx[m] = diff1(rdx, AT(qb, m, -2, 0), AT(qb, m, -1, 0), AT(qb, m, 1, 0), AT(qb, m, 2, 0));
-                qy[m] = diff1(rdy, AT(qb, m, 0, -2), AT(qb, m, 0, -1), AT(qb, m, 0, 1), AT(qb, m, 0, 2));
+            if (P::TT) {
+                qx[m] = diff1(kx0, kx1, QT(m, -2, 0), QT(m, -1, 0), QT(m, 1, 0), QT(m, 2, 0));
+                qy[m] = diff1(ky0, ky1, QT(m, 0, -2), QT(m, 0, -1), QT(m, 0, 1), QT(m, 0, 2));
             }
         }
         const DCell c = dcell(a.gamma, Q);
@@ -196,44 +232,44 @@ __global__ void __launch_bounds__(TI * TJ) k_intflux(const IntFluxArgs a)
 #pragma unroll
             for (int m = 0; m < MEQN; m++) {
                 // F = a1 R1 + dt (b1 f1_t) + a2 R2 + dt (b2 f2_t), left to right
-                Fo[m] = Fo[m] + al * AT(fb, m, 0, 0) + a.dt * (be * -ft[m]);
-                Go[m] = Go[m] + al * AT(gb, m, 0, 0) + a.dt * (be * -gt[m]);
+                Fo[m] = Fo[m] + al * FT(m, 0, 0) + a.dt * (be * -ft[m]);
+                Go[m] = Go[m] + al * GT(m, 0, 0) + a.dt * (be * -gt[m]);
             }
         } else {
             double ftt[MEQN] = {0, 0, 0, 0, 0}, gtt[MEQN] = {0, 0, 0, 0, 0};
-            if (MODE == 1 || MODE == 3) {
+            if (P::TT) {
                 double h1[MEQN], h2[MEQN], fpg[MEQN], v1[MEQN], v2[MEQN], t1[MEQN], t2[MEQN];
                 const DVar vx = dvar(a.gamma, c, qx), vy = dvar(a.gamma, c, qy);
                 dflux2(a.gamma, 1, c, qx, vx, w, vw, h1);
                 dflux2(a.gamma, 2, c, qy, vy, w, vw, h2);
+                const double rdx2 = rdx * rdx, rdy2 = rdy * rdy, m0 = 0.25 * (rdx * rdy), m1 = -(1.0 / 24.0) * (rdx * rdy);
+                const double lx0 = rdx2 * (-1.0 / 12.0), lx1 = rdx2 * (4.0 / 3.0), lx2 = rdx2 * (-5.0 / 2.0);
+                const double ly0 = rdy2 * (-1.0 / 12.0), ly1 = rdy2 * (4.0 / 3.0), ly2 = rdy2 * (-5.0 / 2.0);
 #pragma unroll
                 for (int m = 0; m < MEQN; m++) {
-                    const double fxx = diff2(rdx * rdx, AT(fb, m, -2, 0), AT(fb, m, -1, 0), AT(fb, m, 0, 0),
-                                             AT(fb, m, 1, 0), AT(fb, m, 2, 0));
-                    const double gyy = diff2(rdy * rdy, AT(gb, m, 0, -2), AT(gb, m, 0, -1), AT(gb, m, 0, 0),
-                                             AT(gb, m, 0, 1), AT(gb, m, 0, 2));
-                    double fxy, gxy;
+                    const double fxx = diff2(lx0, lx1, lx2, FT(m, -2, 0), FT(m, -1, 0), FT(m, 0, 0), FT(m, 1, 0),
+                                             FT(m, 2, 0));
+                    const double gyy = diff2(ly0, ly1, ly2, GT(m, 0, -2), GT(m, 0, -1), GT(m, 0, 0), GT(m, 0, 1),
+                                             GT(m, 0, 2));
                     if (MODE == 3) {
                         // 4th-order mixed derivative of LocalIntegrate, ConstructIntegratedR.cpp:427-442
-                        auto mixed = [&](const double* r) {
-                            double t = 0.25 * (AT(r, m, 1, 1) - AT(r, m, -1, 1) - AT(r, m, 1, -1) + AT(r, m, -1, -1));
-                            t -= (1. / 24.) * (AT(r, m, 2, 1) + AT(r, m, -2, -1) - AT(r, m, 2, -1) - AT(r, m, -2, 1) -
-                                               AT(r, m, 1, 2) - AT(r, m, -1, -2) + AT(r, m, 1, -2) + AT(r, m, -1, 2));
-                            return t * (1. / (a.dx * a.dy));
+                        auto mixed = [&](int r, double d2) {
+                            const double t = (QT(r, 1, 1) - QT(r, -1, 1)) - (QT(r, 1, -1) - QT(r, -1, -1));
+                            const double s = ((QT(r, 2, 1) - QT(r, 1, 2)) + (QT(r, -2, -1) - QT(r, -1, -2))) -
+                                             ((QT(r, 2, -1) - QT(r, 1, -2)) + (QT(r, -2, 1) - QT(r, -1, 2)));
+                            return fma(m0, t, fma(m1, s, d2));
                         };
-                        fxy = mixed(fb);
-                        gxy = mixed(gb);
+                        v1[m] = mixed(P::g(m), fxx);
+                        v2[m] = mixed(P::f(m), gyy);
                     } else {
                         // 2nd-order mixed derivative, ConstructIntegratedR.cpp:204-211
-                        fxy = 0.5 * (AT(fb, m, 1, 1) - AT(fb, m, -1, 1)) * rdx;
-                        fxy -= 0.5 * (AT(fb, m, 1, -1) - AT(fb, m, -1, -1)) * rdx;
-                        fxy *= 0.5 * rdy;
-                        gxy = 0.5 * (AT(gb, m, 1, 1) - AT(gb, m, -1, 1)) * rdx;
-                        gxy -= 0.5 * (AT(gb, m, 1, -1) - AT(gb, m, -1, -1)) * rdx;
-                        gxy *= 0.5 * rdy;
+                        auto mixed = [&](int r, double d2) {
+                            const double t = (QT(r, 1, 1) - QT(r, -1, 1)) - (QT(r, 1, -1) - QT(r, -1, -1));
+                            return fma(m0, t, d2);
+                        };
+                        v1[m] = mixed(P::g(m), fxx);
+                        v2[m] = mixed(P::f(m), gyy);
                     }
-                    v1[m] = fxx + gxy;
-                    v2[m] = fxy + gyy;
                 }
                 const DVar v1v = dvar(a.gamma, c, v1), v2v = dvar(a.gamma, c, v2);
                 dflux1(1, c, v1, v1v, t1);
@@ -256,18 +292,20 @@ __global__ void __launch_bounds__(TI * TJ) k_intflux(const IntFluxArgs a)
 #pragma unroll
                 for (int m = 0; m < MEQN; m++) {
                     // ConstructIntegratedR.cpp:685-692, left to right
-                    Fo[m] = Fo[m] + al * AT(fb, m, 0, 0) + a.dt * (be * -ft[m] + ch * a.dt * ftt[m]);
-                    Go[m] = Go[m] + al * AT(gb, m, 0, 0) + a.dt * (be * -gt[m] + ch * a.dt * gtt[m]);
+                    Fo[m] = Fo[m] + al * FT(m, 0, 0) + a.dt * (be * -ft[m] + ch * a.dt * ftt[m]);
+                    Go[m] = Go[m] + al * GT(m, 0, 0) + a.dt * (be * -gt[m] + ch * a.dt * gtt[m]);
                 }
             } else {
 #pragma unroll
                 for (int m = 0; m < MEQN; m++) {
-                    Fo[m] = AT(fb, m, 0, 0) + 0.5 * a.dt * (-ft[m] + a.dt / 3.0 * ftt[m]);
-                    Go[m] = AT(gb, m, 0, 0) + 0.5 * a.dt * (-gt[m] + a.dt / 3.0 * gtt[m]);
+                    Fo[m] = FT(m, 0, 0) + 0.5 * a.dt * (-ft[m] + a.dt / 3.0 * ftt[m]);
+                    Go[m] = GT(m, 0, 0) + 0.5 * a.dt * (-gt[m] + a.dt / 3.0 * gtt[m]);
                 }
             }
         }
-#undef AT
+#undef QT
+#undef FT
+#undef GT
     }
     if (out_ok) {
         const size_t o = size_t(i + 3) * (a.my + 6) + (j + 3);

@@ -665,7 +665,7 @@ int check_status(fin_solver* s)
 
 // ConstructIntegratedR into s->Fg, s->Gg: mode 0/1 = 1-state without/with
 // the f_tt terms, 2 = 2-state.
-constexpr int IF_TI = 16, IF_TJ = 16;
+constexpr int IF_TI = 8, IF_TJ = 16;
 int launch_intflux(fin_solver* s, int mode, const double* q1, const double* q2, double dt, double a1,
                    double b1, double a2, double b2, double c1 = 0.0, double c2 = 0.0)
 {
@@ -678,14 +678,17 @@ int launch_intflux(fin_solver* s, int mode, const double* q1, const double* q2, 
     f.a1 = a1; f.b1 = b1; f.a2 = a2; f.b2 = b2;
     f.c1 = c1; f.c2 = c2;
     f.bc[0] = s->p.bc_xlow; f.bc[1] = s->p.bc_xhigh; f.bc[2] = s->p.bc_ylow; f.bc[3] = s->p.bc_yhigh;
-    constexpr size_t smem = 3 * MEQN * (IF_TI + 4) * (IF_TJ + 4) * sizeof(double);
-    dim3 grid((s->p.my + 6 + IF_TJ - 1) / IF_TJ, (s->p.mx + 6 + IF_TI - 1) / IF_TI);
-    if (mode == 0) k_intflux<0, IF_TI, IF_TJ><<<grid, IF_TI * IF_TJ, smem, s->stream>>>(f);
-    else if (mode == 1) k_intflux<1, IF_TI, IF_TJ><<<grid, IF_TI * IF_TJ, smem, s->stream>>>(f);
-    else if (mode == 2) k_intflux<2, IF_TI, IF_TJ><<<grid, IF_TI * IF_TJ, smem, s->stream>>>(f);
-    else k_intflux<3, IF_TI, IF_TJ><<<grid, IF_TI * IF_TJ, smem, s->stream>>>(f);
+    const dim3 grid((s->p.my + 6 + IF_TJ - 1) / IF_TJ, (s->p.mx + 6 + IF_TI - 1) / IF_TI);
+    auto launch = [&](auto m) {
+        constexpr int MODE = decltype(m)::value;
+        constexpr size_t smem = IntFluxPlanes<MODE>::N * (IF_TI + 4) * (IF_TJ + 4) * sizeof(double);
+        return launch_pdl(k_intflux<MODE, IF_TI, IF_TJ>, grid, dim3(IF_TI * IF_TJ), smem, s->stream, f);
+    };
+    if (mode == 0) CK(launch(std::integral_constant<int, 0>{}));
+    else if (mode == 1) CK(launch(std::integral_constant<int, 1>{}));
+    else if (mode == 2) CK(launch(std::integral_constant<int, 2>{}));
+    else CK(launch(std::integral_constant<int, 3>{}));
     s->launches++;
-    CK(cudaGetLastError());
     return FIN_OK;
 }
 
