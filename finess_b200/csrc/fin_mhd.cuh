@@ -711,6 +711,7 @@ struct MhdDir {
 template <class R, int VER, bool P2, class Cfg, bool HYB = false>
 __global__ void __launch_bounds__(Cfg::NT, Cfg::MINB) k_mhd_stage(const __grid_constant__ MhdArgs a)
 {
+    grid_dependency();
     constexpr int TI = Cfg::TI, TJ = Cfg::TJ, NT = Cfg::NT, H = Cfg::H;
     constexpr int RI = Cfg::RI, RJ = Cfg::RJ, PQ = RI * RJ;
     constexpr int PI = Cfg::PI, PJ = Cfg::PJ, PP = PI * PJ;
