@@ -417,21 +417,23 @@ int launch_stage_cfg(fin_solver* s, const StageArgs& a)
     return FIN_OK;
 }
 
-// FP64 grids of at most SMALL tiles of 15 x 16 leave SMs idle or give some of
-// them twice the work of others: tiles of 7 x 16 with a thread for every face
-// (one round instead of two) spread them.  Twenty steps, us, 15 x 16 / 7 x 16
-// (with five memsets and a copy a step): 64^2 980 / 872, 128^2 990 / 953, 160^2 1002 /
-// 1002, 200^2 (182 tiles) 1249 / 1206; from 256^2 (288) on the larger tile wins,
-// 1260 / 1443.
-constexpr int SMALL = 200;
+// Grids of few tiles of 15 x 16 leave SMs idle or give some of them twice the
+// work of others: tiles of 7 x 16 with a thread for every face (one round instead
+// of two) spread them.  Twenty steps, us, 15 x 16 / 7 x 16:
+//   FP64 (with five memsets and a copy a step), up to SMALL64 tiles: 64^2 980 /
+//   872, 128^2 990 / 953, 160^2 1002 / 1002, 200^2 (182 tiles) 1249 / 1206; from
+//   256^2 (288) on the larger tile wins, 1260 / 1443;
+//   FP32, whose tile is shorter against the launch, while twice the tiles are at
+//   most one an SM: 32^2 607 / 517, 112^2 (56) 604 / 526, 128^2 (72) 607 / 572;
+//   144^2 (90) 607 / 604, 176^2 606 / 656, 320^2 918 / 1076.
+constexpr int SMALL64 = 200, SMALL32 = 74;
 using SmallCfg = TileCfg<7, 16, 256>;
 
 template <class R, int VER, bool P2, bool FG = false>
 int launch_stage_t(fin_solver* s, const StageArgs& a)
 {
     const long long tiles = (long long)((a.mx + Cfg::TI - 1) / Cfg::TI) * ((a.my + Cfg::TJ - 1) / Cfg::TJ);
-    if constexpr (sizeof(R) == 8)
-        if (tiles <= SMALL) return launch_stage_cfg<R, VER, P2, FG, SmallCfg>(s, a);
+    if (tiles <= (sizeof(R) == 8 ? SMALL64 : SMALL32)) return launch_stage_cfg<R, VER, P2, FG, SmallCfg>(s, a);
     return launch_stage_cfg<R, VER, P2, FG, Cfg>(s, a);
 }
 

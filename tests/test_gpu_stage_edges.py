@@ -14,7 +14,7 @@ import pytest
 
 from conftest import interior, rel_linf
 from finess_b200 import problems as P
-from finess_b200._abi import FIN_TS_LXW, FIN_TS_MD, FIN_WENO_FD, FIN_WENO_JS, FIN_WENO_Z
+from finess_b200._abi import FIN_PREC_FP32, FIN_TS_LXW, FIN_TS_MD, FIN_WENO_FD, FIN_WENO_JS, FIN_WENO_Z
 
 pytestmark = pytest.mark.gpu
 
@@ -47,6 +47,27 @@ def test_construct_l_and_step_at_tile_edges(oracle, mx, my, periodic, weno, powe
                                             (195, 240, True)])
 def test_either_side_of_the_tile_rule(oracle, mx, my, periodic, weno, power):
     _check(oracle, mx, my, periodic, weno, power)
+
+
+# FP32 stages turn at 74 tiles of 15 x 16: grids of 74, 75, 72 and 1.  A step of
+# dt = 0.05 h adds twelve face fluxes of weight 0.05, each within some twenty
+# roundings (1.2e-6) of its scale, which is below ten times the state's: 1e-5.
+@pytest.mark.parametrize("weno,power", [(FIN_WENO_JS, 2.0), (FIN_WENO_Z, 2.0), (FIN_WENO_FD, 2.0), (FIN_WENO_Z, 1.5)])
+@pytest.mark.parametrize("mx,my,periodic", [(30, 592, True), (45, 391, False), (128, 128, True), (7, 16, True)])
+def test_either_side_of_the_fp32_tile_rule(oracle, mx, my, periodic, weno, power):
+    from finess_b200.solver import Solver
+    rng = np.random.default_rng(100 * mx + my)
+    p, q = _problem(mx, my, periodic, weno, power, mx % 2 == 0, rng)
+    q = oracle.set_bnd(p, q)
+    dt = 0.05 * min((p.xhigh - p.xlow) / mx, (p.yhigh - p.ylow) / my)
+    qo, cflo = oracle.step_fixed(p, q, dt)
+    p.precision = FIN_PREC_FP32
+    with Solver(p) as s:
+        s.set_state(q)
+        cfl = s.step_fixed(dt)
+        q1, _ = s.get_state()
+    assert rel_linf(interior(p, q1), interior(p, qo)) <= 1e-5
+    assert abs(cfl - cflo) <= 1e-5 * cflo
 
 
 @pytest.mark.parametrize("method,time_order", [(FIN_TS_MD, 4), (FIN_TS_LXW, 3)])
