@@ -13,11 +13,12 @@
 //     time and the speed computed twice (spills 118 -> 8 bytes a thread, and
 //     one-instruction maxima).
 // Layout and schedule, for B200:
-//   * one TI x TJ tile per CTA, three CTAs (24 warps) per SM;
+//   * one TI x TJ tile per CTA, four CTAs (32 warps) per SM (three: 30.7 ->
+//     32.2 ms for the steps above);
 //   * q_in's tile + halo arrives by one TMA copy (tiles clear of the domain
-//     boundary) into an FP64 staging tile that the update reads again for
-//     q_in's interior; the other stage operand's interior arrives by a second
-//     TMA copy that lands while the faces are computed;
+//     boundary) into an FP64 staging tile, whose space the face fluxes take
+//     afterwards; the update reads both stage operands from L2, the one that is
+//     not q_in prefetched into it;
 //   * per cell the half flux and the state are stored as (0.5 f, q) pairs
 //     along each stencil direction, so one 8-byte load serves both terms of
 //     the split; the cell primitives (u, v, p, c) are one 16-byte load;
