@@ -1451,8 +1451,9 @@ int fin_construct_l(fin_solver* s, const double* q_host, double* L_host, double*
 // from the per-face speeds, then the status word.  Both are laid out on the
 // device, so the host moves whole rows: L's packed cells go to q[buf] (the input
 // state, read by now, of the same size), smax to the staging buffer.  300 x 257
-// with both: 1650 -> 740 us (a first call on a solver 4.3 -> 2.6 ms), 1000 x 1100: 35 -> 12 ms (planes copied into a
-// zeroed vector and transposed by the host before).
+// with both: 1650 -> 740 us (a first call on a solver 4.3 -> 2.6 ms), 1000 x
+// 1100: 35 -> 12 ms (planes copied into a zeroed vector and transposed by the
+// host before).
 static int download_l_smax(fin_solver* s, int buf, int outb, double* L_host, double* smax_host)
 {
     const fin_params& p = s->p;
