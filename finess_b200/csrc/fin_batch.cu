@@ -370,18 +370,25 @@ __device__ __forceinline__ void walk_queue(const BProb* pr, const int* act, cons
     const long long total = tile0[na];
     if (threadIdx.x == 0) s_tile = (long long)atomicAdd(queue, 1ull);
     __syncthreads();
-    long long t = s_tile;
+    long long t = s_tile, first = 0, end = 0;   // tiles of the entry lo, problem p
+    int lo = -1, p = 0, tj = 1;
     while (t < total) {
         unsigned long long nx = 0;
         if (threadIdx.x == 0) nx = atomicAdd(queue, 1ull);
-        int lo = 0, hi = na - 1;   // the entry whose tiles contain t
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (tile0[mid] <= t) lo = mid;
-            else hi = mid - 1;
+        if (t >= end) {   // the counter only grows: a later entry
+            int hi = na - 1;
+            lo++;
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (tile0[mid] <= t) lo = mid;
+                else hi = mid - 1;
+            }
+            first = tile0[lo];
+            end = tile0[lo + 1];
+            p = act[lo];
+            tj = (pr[p].my + TJ - 1) / TJ;
         }
-        const int p = act[lo];
-        const int lt = int(t - tile0[lo]), tj = (pr[p].my + TJ - 1) / TJ;
+        const int lt = int(t - first);
         if (!body(p, (lt / tj) * TI, (lt % tj) * TJ)) return;
         __syncthreads();   // the tile's shared memory and s_tile are free
         if (threadIdx.x == 0) s_tile = (long long)nx;
@@ -390,14 +397,33 @@ __device__ __forceinline__ void walk_queue(const BProb* pr, const int* act, cons
     }
 }
 
+// Problem p's stage arguments in shared memory, copied when a CTA comes to its
+// first tile of the problem (no tile is in work then).  With the search of
+// walk_queue only where a CTA leaves a problem's tiles, against arguments read
+// from global memory and a search a tile: a batch of 48 problems (64^2 to 512^2)
+// 159.4 -> 153 ms in FP64, 101.4 -> 96 in FP32; hybrid stages 65.1 -> 63.7.
+__device__ __forceinline__ void take_args(StageArgs& s, const StageArgs* args, int p, int& have)
+{
+    if (p == have) return;
+    static_assert(sizeof(StageArgs) % 8 == 0, "copied by 8-byte words");
+    const unsigned long long* src = reinterpret_cast<const unsigned long long*>(args + p);
+    for (int e = threadIdx.x; e < int(sizeof(StageArgs) / 8); e += blockDim.x)
+        reinterpret_cast<unsigned long long*>(&s)[e] = src[e];
+    have = p;
+    __syncthreads();
+}
+
 // One stage over the problems of a queue (stage_tile, the body of k_stage).
 template <class R, int VER, bool P2, class Cfg>
 __global__ void __launch_bounds__(Cfg::NT, MinBlocks<R>::value)
 k_stage_batch(const BProb* pr, const int* act, const long long* tile0, const int* nact, const StageArgs* args,
               unsigned long long* queue)
 {
+    __shared__ StageArgs a;
+    int have = -1;
     walk_queue<Cfg::TI, Cfg::TJ>(pr, act, tile0, nact, queue, [&](int p, int i0, int j0) {
-        stage_tile<R, VER, P2, Cfg>(args[p], i0, j0);
+        take_args(a, args, p, have);
+        stage_tile<R, VER, P2, Cfg>(a, i0, j0);
         return true;
     });
 }
@@ -410,10 +436,13 @@ __global__ void __launch_bounds__(Cfg::NT, FIN_HYB_CTAS)
 k_stage_hyb_batch(const BProb* pr, const int* act, const long long* tile0, const int* nact, const StageArgs* args,
                   unsigned long long* queue)
 {
+    __shared__ StageArgs a;
+    int have = -1;
     uint32_t phase = 0;
     hyb_mbar_init<Cfg>();
     walk_queue<Cfg::TI, Cfg::TJ>(pr, act, tile0, nact, queue, [&](int p, int i0, int j0) {
-        stage_hyb_tile<VER, P2, Cfg>(args[p], i0, j0, phase);
+        take_args(a, args, p, have);
+        stage_hyb_tile<VER, P2, Cfg>(a, i0, j0, phase);
         tc::fence_smem_to_async();   // the next tile's copy lands where this tile's face fluxes were stored
         return true;
     });
