@@ -8,7 +8,8 @@
 // Two kernels, one thread per cell of a 16 x 16 tile whose states and fluxes
 // sit in shared memory (each cell's three divisions once, not once per face
 // and component: the update kernel 0.130 -> 0.071 ms at 1023 x 1025; both are
-// now bound by the latency of their flux loads):
+// now bound by the latency of their flux loads); launched while their predecessor
+// ends, which takes two steps at 64 x 80 from 92 to 85 us, 1023 x 1025 836 -> 826:
 //   k_mpp_limit   the cell's four limiting factors amin[k] (k = left, right,
 //                 bottom, top face): the density step (:57-92) and the
 //                 pressure step over the 16 on/off combinations of the faces
@@ -206,6 +207,7 @@ __device__ __noinline__ void pressure_step(const MppArgs& a, const Tile& T, int 
 // for bit.  Cells that fail the test (near-vacuum ones) take pressure_step.
 __global__ void __launch_bounds__(NT, 4) k_mpp_limit(const MppArgs a)
 {
+    grid_dependency();
     __shared__ Tile T;
     const int mx = a.mx, my = a.my;
     const int i0 = int(blockIdx.y) * TI, j0 = int(blockIdx.x) * TJ;
@@ -277,6 +279,7 @@ __global__ void __launch_bounds__(NT, 4) k_mpp_limit(const MppArgs a)
 
 __global__ void __launch_bounds__(NT) k_mpp_update(const MppArgs a)
 {
+    grid_dependency();
     __shared__ Tile T;
     __shared__ double red[2][NT / 32];
     const int mx = a.mx, my = a.my;

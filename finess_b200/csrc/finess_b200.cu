@@ -782,8 +782,8 @@ int take_stage_lxw_mpp(fin_solver* s, double dt, int nxt)
     m.alpha_out = alpha_slot(s, nxt);
     m.status = s->status;
     const dim3 blocks((p.my + mpp::TJ - 1) / mpp::TJ, (p.mx + mpp::TI - 1) / mpp::TI);
-    mpp::k_mpp_limit<<<blocks, mpp::NT, 0, s->stream>>>(m);
-    mpp::k_mpp_update<<<blocks, mpp::NT, 0, s->stream>>>(m);
+    CK(launch_pdl(mpp::k_mpp_limit, blocks, dim3(mpp::NT), 0, s->stream, m));
+    CK(launch_pdl(mpp::k_mpp_update, blocks, dim3(mpp::NT), 0, s->stream, m));
     s->launches += 2;
     CK(cudaGetLastError());
     return FIN_OK;
