@@ -11,29 +11,30 @@ namespace fin {
 // of the 260 that a copy through the ring takes).  Plain stores: the page that a
 // fault has just cleared is in the cache, and streaming stores throw it out (345 ->
 // 520 us).  An array whose pages are there already is better left to the runtime's
-// own copy (217 against 250 us), as are copies to the device.  Chunks of 256 KB
+// own copy (217 against 250 us), as are copies to the device.  Chunks of 128 KB
 // (64 KB: 450 us); helper threads fault against one another (4: 800 us).
 struct HostRing {
-    static constexpr size_t CHUNK = size_t(256) << 10;
+    static constexpr size_t CHUNK = size_t(128) << 10;
     static constexpr int N = 4;
-    char* buf;   // BYTES of pinned memory; the events are null at first: the owner is zeroed
+    char* buf;   // null, like the events, at first: the owner is zeroed
     cudaEvent_t ev[N];
 
-    // The pinned bytes are part of an allocation that the owner makes anyway (a
-    // pinned allocation takes 2.5 ms whether it is of 4 KB or of 1 MB).
-    static constexpr size_t BYTES = N * CHUNK;
-
+    // Half a megabyte comes out of the pinned block that holds the owner's step
+    // results (2 us); from a megabyte on the runtime makes a block of its own for
+    // it (2.5 ms).
     cudaError_t ensure()
     {
+        if (buf) return cudaSuccess;
         for (int k = 0; k < N; k++)
             if (!ev[k]) {
                 const cudaError_t e = cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming);
                 if (e != cudaSuccess) return e;
             }
-        return cudaSuccess;
+        return cudaMallocHost(reinterpret_cast<void**>(&buf), N * CHUNK);
     }
     void destroy()
     {
+        if (buf) cudaFreeHost(buf);
         for (int k = 0; k < N; k++)
             if (ev[k]) cudaEventDestroy(ev[k]);
     }

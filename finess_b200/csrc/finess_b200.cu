@@ -85,7 +85,7 @@ struct fin_solver {
     int cur;                // index of q^n
     double* slots;          // NBLOCK blocks of BLOCK doubles, then SMAX_ALT and DIFF
     unsigned int* status;   // the status word of block cb
-    double* h_slots;        // pinned mirror (NSLOTS doubles and the step number), written by the device; ring's bytes
+    double* h_slots;        // pinned mirror (NSLOTS doubles and the step number), written by the device
     int cb, zb;             // block of the current or last step; the block that is all zero (-1: none)
     int ablk[NBUF];         // block that holds the global wave speeds of each buffer
     unsigned long long seq; // steps published
@@ -1245,10 +1245,8 @@ int fin_create(const fin_params* p, fin_solver** out)
     if ((e = cudaMalloc(&s->slots, NDEV * sizeof(double))) != cudaSuccess) return fail(e, "cudaMalloc slots");
     s->status = reinterpret_cast<unsigned int*>(s->slots + SLOT_STATUS);   // block 0 (cb), all buffers' wave speeds there
     s->zb = 1;
-    if ((e = cudaMallocHost(&s->h_slots, HostRing::BYTES + (NSLOTS + 1) * sizeof(double))) != cudaSuccess)
-        return fail(e, "cudaMallocHost");
+    if ((e = cudaMallocHost(&s->h_slots, (NSLOTS + 1) * sizeof(double))) != cudaSuccess) return fail(e, "cudaMallocHost");
     memset(s->h_slots, 0, (NSLOTS + 1) * sizeof(double));
-    s->ring.buf = reinterpret_cast<char*>(s->h_slots + NSLOTS + 1);
     if ((e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking)) != cudaSuccess) return fail(e, "stream");
     if ((e = cudaEventCreate(&s->ev0)) != cudaSuccess) return fail(e, "event");
     if ((e = cudaEventCreate(&s->ev1)) != cudaSuccess) return fail(e, "event");

@@ -1,5 +1,5 @@
 """ConstructL's results on their way to the host: L and smax come in chunks of
-32,768 doubles that end anywhere in a row, so the grids here put a chunk's end
+16,384 doubles that end anywhere in a row, so the grids here put a chunk's end
 on a row's end, inside rows of either parity, and several chunks in one row.
 L against the oracle at the plain method's bar; smax is max-accumulated into
 what the caller gives, exactly."""
@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 
 
 # smax rows hold 2 (my + 1) doubles, L rows 5 my: 64 x 511 ends chunks of smax
-# with its rows; the rows of 2 x 70001 take 10 (L) and 4 (smax) chunks each.
+# with its rows; the rows of 2 x 70001 take 21 (L) and 8 (smax) chunks each.
 @pytest.mark.parametrize("mx,my", [(64, 511), (131, 257), (301, 263), (2, 70001), (70001, 2)])
 @pytest.mark.parametrize("weno,ga", [(FIN_WENO_JS, 1), (FIN_WENO_Z, 0)])
 def test_construct_l_rows(oracle, mx, my, weno, ga):
