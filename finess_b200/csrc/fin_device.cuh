@@ -32,6 +32,25 @@ __device__ __forceinline__ int bc_remap(int k, int n, int bc_lo, int bc_hi)
     return k;
 }
 
+// Loads of global data that an earlier kernel of the stream wrote.  A kernel
+// launched by launch_pdl (fin_pdl.h) may be resident while that kernel still
+// writes, so these are ordinary coherent loads, ordered behind
+// griddepcontrol.wait (volatile statements keep their order): the non-coherent
+// path (__ldg, ld.global.nc) wants data that is read-only for as long as the
+// reading kernel lives, and the compiler may move its loads ahead of the wait.
+__device__ __forceinline__ double ld_dep(const double* p)
+{
+    double v;
+    asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ unsigned ld_dep(const unsigned* p)
+{
+    unsigned v;
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+
 // Non-negative doubles order like their bit patterns, so an unsigned 64-bit
 // atomicMax is an exact max (NaN with a clear sign bit compares above +Inf,
 // so a NaN wave speed wins the max and is seen by the host).

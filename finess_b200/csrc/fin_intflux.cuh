@@ -175,15 +175,15 @@ __global__ void __launch_bounds__(TI * TJ, IntFluxPlanes<MODE>::CTAS) k_intflux(
                 const int gj = bc_remap(j0 - HB + jj, a.my, a.bc[2], a.bc[3]);
                 const size_t g = size_t(gi) * a.my + gj;
 #pragma unroll
-                for (int m = 0; m < MEQN; m++) Qv[it][m] = __ldg(q + m * a.plane + g);
+                for (int m = 0; m < MEQN; m++) Qv[it][m] = ld_dep(q + m * a.plane + g);
             }
         }
         double Q[MEQN];
         if (!P::TT) {
             const size_t g = size_t(bc_remap(i, a.mx, a.bc[0], a.bc[1])) * a.my + bc_remap(j, a.my, a.bc[2], a.bc[3]);
-            Q[0] = __ldg(q + g);
-            Q[3] = __ldg(q + 3 * a.plane + g);
-            Q[4] = __ldg(q + 4 * a.plane + g);
+            Q[0] = ld_dep(q + g);
+            Q[3] = ld_dep(q + 3 * a.plane + g);
+            Q[4] = ld_dep(q + 4 * a.plane + g);
         }
 #pragma unroll
         for (int it = 0; it < NIT; it++) {

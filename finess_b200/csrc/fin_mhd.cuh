@@ -418,7 +418,7 @@ __device__ __forceinline__ unsigned mask_row_wrapped(const unsigned* row, int nw
 {
     if (c0 >= 0 && c0 + nb <= period) {
         const int k = c0 >> 5;
-        const unsigned lo = __ldg(row + k), hi = k + 1 < nw ? __ldg(row + k + 1) : 0u;
+        const unsigned lo = ld_dep(row + k), hi = k + 1 < nw ? ld_dep(row + k + 1) : 0u;
         return row_bits(lo, hi, c0) & (nb >= 32 ? 0xffffffffu : ((1u << nb) - 1u));
     }
     unsigned m = 0;
@@ -426,7 +426,7 @@ __device__ __forceinline__ unsigned mask_row_wrapped(const unsigned* row, int nw
         int c = c0 + b;
         if (c < 0) c += period;
         else if (c >= period) c -= period;
-        m |= ((__ldg(row + (c >> 5)) >> (c & 31)) & 1u) << b;
+        m |= ((ld_dep(row + (c >> 5)) >> (c & 31)) & 1u) << b;
     }
     return m;
 }
@@ -760,7 +760,7 @@ __global__ void __launch_bounds__(Cfg::NT, Cfg::MINB) k_mhd_stage(const __grid_c
                 const int gj = pwrap(j0 + jj - H, my);
                 const size_t g = size_t(gi) * my + gj;
 #pragma unroll
-                for (int m = 0; m < MHD_NQ; m++) vq[it][m] = __ldg(a.qin + m * a.plane + g);
+                for (int m = 0; m < MHD_NQ; m++) vq[it][m] = ld_dep(a.qin + m * a.plane + g);
             }
         }
 #pragma unroll
@@ -770,7 +770,7 @@ __global__ void __launch_bounds__(Cfg::NT, Cfg::MINB) k_mhd_stage(const __grid_c
                 const int ii = e / AJ, jj = e - ii * AJ;
                 const int gi = pwrap(i0 + ii - HA, mx);
                 const int gj = pwrap(j0 + jj - HA, my);
-                va[it] = __ldg(a.qin + 8 * a.plane + size_t(gi) * my + gj);
+                va[it] = ld_dep(a.qin + 8 * a.plane + size_t(gi) * my + gj);
             }
         }
 #pragma unroll
@@ -782,8 +782,8 @@ __global__ void __launch_bounds__(Cfg::NT, Cfg::MINB) k_mhd_stage(const __grid_c
             if (e < Cfg::NI * NJ && (xin || yin)) {
                 const size_t g = 8 * a.plane + size_t(pwrap(i0 + ci, mx)) * my + pwrap(j0 + cj, my);
                 double v = 0.0;
-                if (a.A) v = a.a1 * __ldg(a.A + g);
-                if (a.B) v = v + a.a2 * __ldg(a.B + g);
+                if (a.A) v = a.a1 * ld_dep(a.A + g);
+                if (a.B) v = v + a.a2 * ld_dep(a.B + g);
                 vab[it] = v;
             }
         }

@@ -3,6 +3,8 @@
 // griddepcontrol.wait before it reads anything an earlier kernel wrote, and
 // griddepcontrol.launch_dependents so that its own successor may be placed; the
 // wait returns when the kernel ahead has completed and its writes are visible.
+// Such a kernel reads what earlier kernels wrote by plain loads, ld_dep
+// (fin_device.cuh), cp.async or TMA, never through the non-coherent path.
 #pragma once
 #include <cuda_runtime.h>
 

@@ -199,7 +199,7 @@ __device__ __forceinline__ void stage_remap(double* stg, const double* q, size_t
         const int gj = bc_remap(j0 + jj - H, my, bc[2], bc[3]);
         const size_t g = size_t(gi) * my + gj;
 #pragma unroll
-        for (int m = 0; m < MEQN; m++) stg[(m * RI + ii) * Cfg::SJ + jj + 1] = __ldg(q + m * plane + g);
+        for (int m = 0; m < MEQN; m++) stg[(m * RI + ii) * Cfg::SJ + jj + 1] = ld_dep(q + m * plane + g);
     }
 }
 
@@ -641,7 +641,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const int i0, con
             const int gj = bc_remap(j0 + jj - H, my, a.bc[2], a.bc[3]);
             const size_t g = size_t(gi) * my + gj;
 #pragma unroll
-            for (int m = 0; m < MEQN; m++) v[m] = R(__ldg(a.qin + m * a.plane + g));
+            for (int m = 0; m < MEQN; m++) v[m] = R(ld_dep(a.qin + m * a.plane + g));
         };
         auto cell = [&](int e, const R* v) {
             int ii, jj;
@@ -669,12 +669,12 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const int i0, con
                 if (yin) {
                     const int d = ii * FS + (jj - H);
 #pragma unroll
-                    for (int m = 0; m < MEQN; m++) S.fs[m * RI * FS + d] = R(0.5 * __ldg(a.Fg + m * a.gplane + o));
+                    for (int m = 0; m < MEQN; m++) S.fs[m * RI * FS + d] = R(0.5 * ld_dep(a.Fg + m * a.gplane + o));
                 }
                 if (xin) {
                     const int d = (ii - H) * RJ + jj;
 #pragma unroll
-                    for (int m = 0; m < MEQN; m++) S.gs[m * TI * RJ + d] = R(0.5 * __ldg(a.Gg + m * a.gplane + o));
+                    for (int m = 0; m < MEQN; m++) S.gs[m * TI * RJ + d] = R(0.5 * ld_dep(a.Gg + m * a.gplane + o));
                 }
                 return;
             }

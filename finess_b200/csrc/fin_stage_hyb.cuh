@@ -219,8 +219,8 @@ __device__ __forceinline__ void stage_hyb_tile(const StageArgs& a, const int i0,
             if (a1 >= 0 && a1 < mx) { row = a.flags + size_t(mx + 1) * wx + size_t(a1) * wy; nw = wy; }
         }
         if (row) {
-            if (k >= 0 && k < nw) fw_lo = __ldg(row + k);
-            if (k + 1 < nw) fw_hi = __ldg(row + k + 1);
+            if (k >= 0 && k < nw) fw_lo = ld_dep(row + k);
+            if (k + 1 < nw) fw_hi = ld_dep(row + k + 1);
         }
         if (!tt) stage_remap<Cfg>(stg, a.qin, a.plane, i0, j0, mx, my, a.bc, tid);
         if (tid < Cfg::FXR) {
