@@ -914,6 +914,7 @@ int fin_mhd_step_fixed(fin_mhd* s, double dt, double* cfl_out)
     settle_judge(s, nxt, dt, &cfl);
     if (nonfinite) return merr(FIN_ERR_NONFINITE, "non-finite wave speed or state");
     float ms = 0.f;
+    MCK(cudaEventSynchronize(s->ev1));   // read_step waits for its number, not for the event
     MCK(cudaEventElapsedTime(&ms, s->ev0, s->ev1));
     s->last_ms = ms;
     s->cur = nxt;
