@@ -64,9 +64,10 @@ __device__ __forceinline__ void atomic_max_nonneg(double* addr, double v)
 template <class R> __host__ __device__ __forceinline__ R Max(R a, R b) { return a > b ? a : b; }
 template <class R> __host__ __device__ __forceinline__ R Min(R a, R b) { return a < b ? a : b; }
 
-// Maximum and minimum that give NaN when either operand is NaN: one FP32
-// instruction where the comparison forms above take two.  Used for wave
-// speeds, where a NaN comes from a state that the non-finite check reports.
+// Maximum and minimum of wave speeds.  FP32: one instruction where the
+// comparison forms above take two, NaN when either operand is.  FP64: the
+// comparison forms, NaN when the second operand is; a face's second operand
+// comes from both its cells, so a NaN of either reaches the non-finite check.
 __device__ __forceinline__ float MaxN(float a, float b)
 {
     float r;
@@ -181,12 +182,13 @@ __device__ __forceinline__ float rsqrt_fast(float x)
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
-// sqrt(x) for x >= 0 as x / sqrt(x); zero and subnormal x give 0 (compared on
-// the high word, which costs no FP64 instruction), Inf and NaN give NaN.
+// sqrt(x) as x / sqrt(x); zero and subnormal x of either sign give 0 (compared
+// on the high word, which costs no FP64 instruction), negative x, Inf and a NaN
+// of either sign give NaN.
 __device__ __forceinline__ double sqrt_fast(double x)
 {
     const double s = x * rsqrt_fast(x);
-    return __double2hiint(x) < 0x00100000 ? 0.0 : s;
+    return (__double2hiint(x) & 0x7fffffff) < 0x00100000 ? 0.0 : s;
 }
 __device__ __forceinline__ float sqrt_fast(float x) { return fsqrt(x); }
 

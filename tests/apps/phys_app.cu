@@ -98,7 +98,7 @@ struct App : AppBase {
     int step_fixed(double dt, double* cfl) override { return d.step_fixed(dt, cfl); }
 };
 
-// The library's reciprocal (fin_device.cuh: Newton-Raphson refinement of
+// The library's reciprocal (fin_device.cuh: one third-order step from
 // rcp.approx) beside CUDA's correctly rounded division, for a sweep of
 // arguments.
 __global__ void k_rcp_probe(const double* x, double* r64, double* div64, float* r32, int n)
@@ -107,6 +107,20 @@ __global__ void k_rcp_probe(const double* x, double* r64, double* div64, float* 
         r64[k] = fin::rcp(x[k]);
         div64[k] = __ddiv_rn(1.0, x[k]);
         r32[k] = fin::rcp(float(x[k]));
+    }
+}
+
+// The library's square roots of x[k] beside CUDA's correctly rounded one:
+// out[0..2][n] sqrt_fast, rsqrt_fast and __dsqrt_rn, out[3..4][n] sqrt_fast
+// and rsqrt_fast of float(x[k]).
+__global__ void k_root_probe(const double* x, double* out, int n)
+{
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+        out[k] = fin::sqrt_fast(x[k]);
+        out[n + k] = fin::rsqrt_fast(x[k]);
+        out[2 * n + k] = __dsqrt_rn(x[k]);
+        out[3 * n + k] = double(fin::sqrt_fast(float(x[k])));
+        out[4 * n + k] = double(fin::rsqrt_fast(float(x[k])));
     }
 }
 
@@ -133,6 +147,21 @@ int app_rcp_probe(const double* x, double* r64, double* div64, float* r32, int n
     cudaFree(d64);
     cudaFree(dd);
     cudaFree(d32);
+    return rc;
+}
+
+// k_root_probe of n host values, out[5][n].
+int app_root_probe(const double* x, double* out, int n)
+{
+    double *dx = nullptr, *dout = nullptr;
+    if (cudaMalloc(&dx, n * sizeof(double)) != cudaSuccess || cudaMalloc(&dout, 5 * n * sizeof(double)) != cudaSuccess)
+        return FIN_ERR_CUDA;
+    cudaMemcpy(dx, x, n * sizeof(double), cudaMemcpyHostToDevice);
+    k_root_probe<<<(n + 255) / 256, 256>>>(dx, dout, n);
+    int rc = cudaGetLastError() == cudaSuccess ? FIN_OK : FIN_ERR_CUDA;
+    if (cudaMemcpy(out, dout, 5 * n * sizeof(double), cudaMemcpyDeviceToHost) != cudaSuccess) rc = FIN_ERR_CUDA;
+    cudaFree(dx);
+    cudaFree(dout);
     return rc;
 }
 
