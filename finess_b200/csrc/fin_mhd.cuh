@@ -113,12 +113,17 @@ __device__ __forceinline__ float xdiv(float a, float b) { return __fdiv_rn(a, b)
 // through the nonlinear WENO weights the fluxes, follow those rounding bits.
 // The FP64 form therefore evaluates such faces' chain in the reference's order
 // with IEEE operations and no contraction (EXACT), so that it takes the same
-// values; where c_f^2 - a^2, a^2 - c_s^2 and c_s^2 are each above 1e-6 of
+// values; where c_f^2 - a^2, a^2 - c_s^2 and c_s^2 are each above 1e-4 of
 // c_f^2 - c_s^2 (resp. d) and that above 0.05 d the scalars are conditioned
-// well enough (rounding reaches them amplified by at most 1e3, 1e-13, and the
+// well enough (rounding reaches them amplified by about 1e2, 1e-14, and the
 // fluxes only through the nonlinear weights) that the short chain serves: six
 // divisions and six square roots in sequence, about 250 dependent FP64
-// operations, were a seventh of the face's work and its longest latency.  In FP32 the chain breaks down near the umbilic point (B_perp -> 0,
+// operations, were a seventh of the face's work and its longest latency.  The
+// line lies at 1e-4 because the departure from the reference in L, for states
+// whose transverse field falls to 1e-9, is then that of the exact chain at every
+// face (5e-15; 1.4e-14 with the line at 1e-6), for 0.3 % of the step (2.489
+// against 2.481 ms, two steps at 1024^2; 1e-3: 2.503).
+// In FP32 the chain breaks down near the umbilic point (B_perp -> 0,
 // a^2 -> B_n^2/rho): c_f^2 - c_s^2 = sqrt(disc) is resolved to ~3e-4 of d
 // only, alpha_f and alpha_s become 0/0, and left times right eigenvectors
 // departs from the identity (measured: NaN or 2e-4 in FP32, 1e-16 in FP64).
@@ -195,8 +200,8 @@ __device__ __forceinline__ MhdEigScalars<R> mhd_eig_scalars(const MhdArgs& a, R 
     bool umb;
     mhd_eig_core<R, false>(gamma, Q, e, d, umb);
     if constexpr (sizeof(R) == 8) {
-        const R cf2 = e.cf * e.cf, cs2 = e.cs * e.cs, lim = R(1.0e-6) * (cf2 - cs2);
-        if (!(cf2 - e.a2 > lim && e.a2 - cs2 > lim && cs2 > R(1.0e-6) * d && cf2 - cs2 > R(0.05) * d)) {
+        const R cf2 = e.cf * e.cf, cs2 = e.cs * e.cs, lim = R(1.0e-4) * (cf2 - cs2);
+        if (!(cf2 - e.a2 > lim && e.a2 - cs2 > lim && cs2 > R(1.0e-4) * d && cf2 - cs2 > R(0.05) * d)) {
             R q[MHD_NQ];
             MhdEigScalars<R> x;
             bool u;
