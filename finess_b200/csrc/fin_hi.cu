@@ -1,7 +1,7 @@
 // The stage kernel of the spatial orders other than 5 (space_order 1, 7, 9,
 // 11; ConstructL.cpp:31-33, 62-358), FP64: k_stage with a halo of r =
 // (space_order + 1) / 2 cells and the reconstructions of fin_weno_hi.cuh.  A
-// translation unit of its own (13 instantiations).
+// translation unit of its own (26 instantiations).
 //
 // What bounds it: the FP64 pipe, and shared-memory reads of the longer stencils
 // beside it (65 and 76 % busy for WENO7-JS).  Two SSP-RK3 steps at 1024^2, ms,
@@ -17,11 +17,12 @@
 namespace fin {
 namespace hi {
 
-template <int ORDER, int VER, bool P2>
+template <int ORDER, int VER, bool P2, bool LONG = false>
 cudaError_t launch_t(const StageArgs& a, cudaStream_t stream)
 {
     using Cfg = TileCfg<15, 16, 256, (ORDER + 1) / 2>;
-    auto kern = k_stage<double, VER, P2, Cfg, false, ORDER>;
+    if (!LONG && (a.mx + Cfg::TI - 1) / Cfg::TI > 65535) return launch_t<ORDER, VER, P2, true>(a, stream);
+    auto kern = k_stage<double, VER, P2, Cfg, false, ORDER, LONG>;
     const size_t smem = Cfg::template smem_bytes<double>();
     static bool configured = false;   // per instantiation; the attribute is per device function
     if (!configured) {
@@ -29,8 +30,7 @@ cudaError_t launch_t(const StageArgs& a, cudaStream_t stream)
         if (e != cudaSuccess) return e;
         configured = true;
     }
-    const dim3 grid((a.my + Cfg::TJ - 1) / Cfg::TJ, (a.mx + Cfg::TI - 1) / Cfg::TI);
-    return launch_pdl(kern, grid, dim3(Cfg::NT), smem, stream, a);
+    return launch_pdl(kern, tile_grid(a.mx, a.my, Cfg::TI, Cfg::TJ), dim3(Cfg::NT), smem, stream, a);
 }
 
 template <int ORDER>

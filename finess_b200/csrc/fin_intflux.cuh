@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(TI * TJ, IntFluxPlanes<MODE>::CTAS) k_intflux(
     double* sb = reinterpret_cast<double*>(smem_raw);   // [P::N][BI][BJ]
     grid_dependency();
     const int tid = threadIdx.x;
-    const int i0 = int(blockIdx.y) * TI - 3, j0 = int(blockIdx.x) * TJ - 3;   // extended-domain origin
+    const int i0 = tile_row() * TI - 3, j0 = int(blockIdx.x) * TJ - 3;   // extended-domain origin
     const int ci = tid / TJ, cj = tid - ci * TJ;
     const int i = i0 + ci, j = j0 + cj;                // this thread's output cell
     const bool out_ok = i < a.mx + 3 && j < a.my + 3;

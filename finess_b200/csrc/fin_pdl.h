@@ -10,6 +10,18 @@
 
 namespace fin {
 
+// Blocks for tiles of ti x tj cells: columns of tiles in x, rows in y and, as y
+// takes 65,535, the rest in z (tile_row).  The last few rows of tiles may then lie
+// past the grid, like the cells of a partial tile.
+inline dim3 tile_grid(long long mx, long long my, int ti, int tj)
+{
+    const long long rows = (mx + ti - 1) / ti, cols = (my + tj - 1) / tj, z = (rows + 65534) / 65535;
+    return dim3(unsigned(cols), unsigned((rows + z - 1) / z), unsigned(z));
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ int tile_row() { return int(blockIdx.z * gridDim.y + blockIdx.y); }
+#endif
+
 template <class... P, class... A>
 inline cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args)
 {

@@ -49,6 +49,7 @@
 // FP32 form's step from 1.69 to 1.48 ms (two steps of 4001 x 515).
 #pragma once
 #include "fin_device.cuh"
+#include "fin_pdl.h"
 #include "fin_tc.cuh"
 #include "fin_weno_face.cuh"
 #include "fin_weno_hi.cuh"
@@ -827,12 +828,16 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, const int i0, con
     }
 }
 
-template <class R, int VER, bool P2, class Cfg, bool FG = false, int ORDER = 5>
+// LONG: rows of tiles in blockIdx.y and .z (tile_grid), for grids of more than
+// 65,535 rows of tiles; a kernel of its own, as the row's index costs a register
+// that the orders above 5 have not got (WENO7-JS 1.477 -> 1.543 ms, two steps
+// at 1024^2).
+template <class R, int VER, bool P2, class Cfg, bool FG = false, int ORDER = 5, bool LONG = false>
 __global__ void __launch_bounds__(Cfg::NT, MinBlocks<R>::value * 256 / Cfg::NT) k_stage(const __grid_constant__ StageArgs a)
 {
     grid_dependency();
     static_assert(ORDER == 5 ? Cfg::H == 3 : Cfg::H == (ORDER + 1) / 2 && sizeof(R) == 8 && !FG, "halo of the stencil");
-    stage_tile<R, VER, P2, Cfg, FG, ORDER>(a, blockIdx.y * Cfg::TI, blockIdx.x * Cfg::TJ);
+    stage_tile<R, VER, P2, Cfg, FG, ORDER>(a, (LONG ? tile_row() : int(blockIdx.y)) * Cfg::TI, blockIdx.x * Cfg::TJ);
 }
 
 // GlobalWaveSpd (lib/2d/GlobalWaveSpd.cpp:52-78) on a state already in HBM:

@@ -680,7 +680,7 @@ int launch_intflux(fin_solver* s, int mode, const double* q1, const double* q2, 
     f.a1 = a1; f.b1 = b1; f.a2 = a2; f.b2 = b2;
     f.c1 = c1; f.c2 = c2;
     f.bc[0] = s->p.bc_xlow; f.bc[1] = s->p.bc_xhigh; f.bc[2] = s->p.bc_ylow; f.bc[3] = s->p.bc_yhigh;
-    const dim3 grid((s->p.my + 6 + IF_TJ - 1) / IF_TJ, (s->p.mx + 6 + IF_TI - 1) / IF_TI);
+    const dim3 grid = tile_grid(s->p.mx + 6, s->p.my + 6, IF_TI, IF_TJ);
     auto launch = [&](auto m) {
         constexpr int MODE = decltype(m)::value;
         constexpr size_t smem = IntFluxPlanes<MODE>::N * (IF_TI + 4) * (IF_TJ + 4) * sizeof(double);
