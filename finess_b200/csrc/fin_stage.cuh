@@ -294,12 +294,12 @@ __device__ __forceinline__ R weno_pair(R* dp, R* dm, R eps4, R pw)
 }
 
 // A correction of another order, fenced.
-template <int ORDER, int VER, bool P2>
+template <int ORDER, int VER, bool P2, bool CALL>
 __device__ __forceinline__ double hi_fenced(double* d, double eps, double pw)
 {
 #pragma unroll
     for (int k = 0; k < ORDER - 1; k++) fence(d[k]);
-    double c = hi::correction<ORDER, VER, P2>(d, eps, pw);
+    double c = hi::correction<ORDER, VER, P2, CALL>(d, eps, pw);
     fence(c);
     return c;
 }
@@ -447,6 +447,7 @@ __device__ __forceinline__ R stage_face(const StageArgs& a, const StageSmem<R, C
         // 0 .. ORDER-1, gm from v- at the points ORDER .. 1 -- fields 0, 1 and
         // 4, then 2 and 3; the fields' sums wait in the face's flux slots.
         constexpr int NW = ORDER, C = (ORDER - 1) / 2;   // points, the upwind one
+        constexpr bool CALL = Cfg::ONE_ROUND || VER == FIN_WENO_Z;
         auto half = [&](auto minus) {
             constexpr bool M = decltype(minus)::value;
             const R l = M ? -lah : lah;
@@ -469,9 +470,9 @@ __device__ __forceinline__ R stage_face(const StageArgs& a, const StageSmem<R, C
                     if (t == C) { put(0, w0); put(1, w1); put(4, w4); }
                     c0 = w0; c1 = w1; c4 = w4;
                 }
-                out[0] += hi_fenced<ORDER, VER, P2>(d0, eps, pw);
-                out[4 * OP] += hi_fenced<ORDER, VER, P2>(d4, eps, pw);
-                out[OP] += hi_fenced<ORDER, VER, P2>(d1, eps, pw);
+                out[0] += hi_fenced<ORDER, VER, P2, CALL>(d0, eps, pw);
+                out[4 * OP] += hi_fenced<ORDER, VER, P2, CALL>(d4, eps, pw);
+                out[OP] += hi_fenced<ORDER, VER, P2, CALL>(d1, eps, pw);
             }
             {
                 R d2[NW], d3[NW], c2, c3;
@@ -486,8 +487,8 @@ __device__ __forceinline__ R stage_face(const StageArgs& a, const StageSmem<R, C
                     if (t == C) { put(2, w2); put(3, w3); }
                     c2 = w2; c3 = w3;
                 }
-                out[2 * OP] += hi_fenced<ORDER, VER, P2>(d2, eps, pw);
-                out[3 * OP] += hi_fenced<ORDER, VER, P2>(d3, eps, pw);
+                out[2 * OP] += hi_fenced<ORDER, VER, P2, CALL>(d2, eps, pw);
+                out[3 * OP] += hi_fenced<ORDER, VER, P2, CALL>(d3, eps, pw);
             }
         };
         half(std::false_type{});

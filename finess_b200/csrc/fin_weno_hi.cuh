@@ -137,8 +137,17 @@ template <> struct Scheme<11> {
     __device__ __forceinline__ static double tau(const double* x) { return 0.; }   // no Z weights of this order
 };
 
+// Powers other than 2 (CALL: one copy of pow instead of one a weight; which
+// is better where is measured at fin_hi.cu's launch_t).
+static __device__ __noinline__ double pow_call(double x, double p) { return pow(x, p); }
+template <bool CALL>
+__device__ __forceinline__ double power(double x, double p)
+{
+    return CALL ? pow_call(x, p) : pow(x, p);
+}
+
 // The reconstruction of order ORDER minus its upwind point u_i.
-template <int ORDER, int VER, bool P2>
+template <int ORDER, int VER, bool P2, bool CALL>
 __device__ __forceinline__ double correction(const double* d, double eps, double pw)
 {
     static_assert(ORDER == 1 || ORDER == 7 || ORDER == 9 || ORDER == 11, "orders 1, 7, 9, 11");
@@ -167,7 +176,7 @@ __device__ __forceinline__ double correction(const double* d, double eps, double
                     const double r = VER == FIN_WENO_Z ? tau * rcp(x[k]) : rcp(x[k]);
                     w = VER == FIN_WENO_Z ? fma(r, r, 1.0) : r * r;
                 } else {
-                    w = VER == FIN_WENO_Z ? 1.0 + pow(tau / x[k], pw) : pow(x[k], -pw);
+                    w = VER == FIN_WENO_Z ? 1.0 + power<CALL>(tau / x[k], pw) : power<CALL>(x[k], -pw);
                 }
                 w *= S::weight(k);
                 num = fma(w, c[k], num);
