@@ -6,8 +6,10 @@ namespace fin {
 struct StageArgs;
 namespace hi {
 
-// One stage of space_order 1, 7, 9 or 11 with the given WENO version (power2:
-// power_param is 2); cudaErrorInvalidValue for a pair that is not built.
+inline bool built(int order) { return order == 1 || order == 7 || order == 9 || order == 11; }
+
+// One stage of a space_order that is built, with the given WENO version (power2:
+// power_param is 2).
 cudaError_t launch(int order, int weno_version, bool power2, const StageArgs& a, cudaStream_t stream);
 
 }  // namespace hi

@@ -506,9 +506,8 @@ int launch_stage_hyb(fin_solver* s, const StageArgs& a)
 // Spatial orders other than 5 (FP64): instantiated in fin_hi.cu.
 int launch_stage_hi(fin_solver* s, const StageArgs& a)
 {
-    const cudaError_t e = fin::hi::launch(s->p.space_order, s->p.weno_version, s->p.power_param == 2.0, a, s->stream);
-    if (e == cudaErrorInvalidValue) return set_err(FIN_ERR_ARG, "Requested WENO Reconstruction not implemented.");
-    CK(e);
+    if (!fin::hi::built(s->p.space_order)) return set_err(FIN_ERR_ARG, "Requested WENO Reconstruction not implemented.");
+    CK(fin::hi::launch(s->p.space_order, s->p.weno_version, s->p.power_param == 2.0, a, s->stream));
     s->launches++;
     return FIN_OK;
 }
