@@ -46,52 +46,48 @@ inline bool small_tile(long long tiles)
 }
 
 template <int ORDER, int VER, bool P2, bool SMALL, bool LONG = false>
-cudaError_t launch_tile(const StageArgs& a, cudaStream_t stream)
+cudaError_t launch_tile(const StageArgs& a, SmemGrants& g, cudaStream_t stream)
 {
     using Cfg = TileCfg<(SMALL ? 7 : 15), 16, 256, (ORDER + 1) / 2>;
     if constexpr (!LONG && (!SMALL || ORDER == 11)) {
-        if ((a.mx + Cfg::TI - 1) / Cfg::TI > 65535) return launch_tile<ORDER, VER, P2, SMALL, true>(a, stream);
+        if ((a.mx + Cfg::TI - 1) / Cfg::TI > 65535) return launch_tile<ORDER, VER, P2, SMALL, true>(a, g, stream);
     }
     auto kern = k_stage<double, VER, P2, Cfg, false, ORDER, LONG>;
     const size_t smem = Cfg::template smem_bytes<double>();
-    static bool configured = false;   // per instantiation; the attribute is per device function
-    if (!configured) {
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-        if (e != cudaSuccess) return e;
-        configured = true;
-    }
+    const cudaError_t e = g.allow(kern, smem);
+    if (e != cudaSuccess) return e;
     return launch_pdl(kern, tile_grid(a.mx, a.my, Cfg::TI, Cfg::TJ), dim3(Cfg::NT), smem, stream, a);
 }
 
 template <int ORDER, int VER, bool P2>
-cudaError_t launch_t(const StageArgs& a, cudaStream_t stream)
+cudaError_t launch_t(const StageArgs& a, SmemGrants& g, cudaStream_t stream)
 {
     if constexpr (P2) {
-        return launch_tile<ORDER, VER, P2, false>(a, stream);
+        return launch_tile<ORDER, VER, P2, false>(a, g, stream);
     } else if constexpr (ORDER == 11) {
-        return launch_tile<ORDER, VER, P2, true>(a, stream);
+        return launch_tile<ORDER, VER, P2, true>(a, g, stream);
     } else {
         const long long tiles = (long long)((a.mx + 14) / 15) * ((a.my + 15) / 16);
-        return small_tile(tiles) ? launch_tile<ORDER, VER, P2, true>(a, stream)
-                                 : launch_tile<ORDER, VER, P2, false>(a, stream);
+        return small_tile(tiles) ? launch_tile<ORDER, VER, P2, true>(a, g, stream)
+                                 : launch_tile<ORDER, VER, P2, false>(a, g, stream);
     }
 }
 
 template <int ORDER>
-cudaError_t launch_o(int v, bool p2, const StageArgs& a, cudaStream_t s)
+cudaError_t launch_o(int v, bool p2, const StageArgs& a, SmemGrants& g, cudaStream_t s)
 {
-    if (v == FIN_WENO_FD) return launch_t<ORDER, FIN_WENO_FD, true>(a, s);
-    if (v == FIN_WENO_Z) return p2 ? launch_t<ORDER, FIN_WENO_Z, true>(a, s) : launch_t<ORDER, FIN_WENO_Z, false>(a, s);
-    return p2 ? launch_t<ORDER, FIN_WENO_JS, true>(a, s) : launch_t<ORDER, FIN_WENO_JS, false>(a, s);
+    if (v == FIN_WENO_FD) return launch_t<ORDER, FIN_WENO_FD, true>(a, g, s);
+    if (v == FIN_WENO_Z) return p2 ? launch_t<ORDER, FIN_WENO_Z, true>(a, g, s) : launch_t<ORDER, FIN_WENO_Z, false>(a, g, s);
+    return p2 ? launch_t<ORDER, FIN_WENO_JS, true>(a, g, s) : launch_t<ORDER, FIN_WENO_JS, false>(a, g, s);
 }
 
-cudaError_t launch(int order, int v, bool p2, const StageArgs& a, cudaStream_t s)
+cudaError_t launch(int order, int v, bool p2, const StageArgs& a, SmemGrants& g, cudaStream_t s)
 {
     switch (order) {
-    case 1: return launch_t<1, FIN_WENO_JS, true>(a, s);
-    case 7: return launch_o<7>(v, p2, a, s);
-    case 9: return launch_o<9>(v, p2, a, s);
-    case 11: return p2 ? launch_t<11, FIN_WENO_JS, true>(a, s) : launch_t<11, FIN_WENO_JS, false>(a, s);
+    case 1: return launch_t<1, FIN_WENO_JS, true>(a, g, s);
+    case 7: return launch_o<7>(v, p2, a, g, s);
+    case 9: return launch_o<9>(v, p2, a, g, s);
+    case 11: return p2 ? launch_t<11, FIN_WENO_JS, true>(a, g, s) : launch_t<11, FIN_WENO_JS, false>(a, g, s);
     }
     return cudaErrorInvalidValue;
 }

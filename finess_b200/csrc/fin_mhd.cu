@@ -21,6 +21,7 @@
 #include "fin_mhd.cuh"
 #include "fin_mhd_hyb.cuh"
 #include "fin_pdl.h"
+#include "fin_smem.h"
 
 using namespace fin;
 
@@ -104,6 +105,7 @@ struct fin_mhd {
     double* d_face_x;
     double* d_face_y;
     cudaStream_t stream;
+    SmemGrants smem;
     cudaEvent_t ev0, ev1, kev[6];
     bool time_kernels;
     double kernel_ms;
@@ -353,12 +355,7 @@ int launch_t(fin_mhd* s, const MhdArgs& a)
 {
     using MCfg = typename MCfgOf<R, HYB>::T;
     constexpr size_t smem = HYB ? MCfg::template smem_bytes_hyb<R>() : MCfg::template smem_bytes<R>();
-    static bool attr = false;
-    if (!attr) {
-        MCK(cudaFuncSetAttribute(k_mhd_stage<R, VER, P2, MCfg, HYB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(smem)));
-        attr = true;
-    }
+    MCK(s->smem.allow(k_mhd_stage<R, VER, P2, MCfg, HYB>, smem));
     dim3 grid((s->p.my + MCfg::TJ - 1) / MCfg::TJ, (s->p.mx + MCfg::TI - 1) / MCfg::TI);
     MCK(launch_pdl(k_mhd_stage<R, VER, P2, MCfg, HYB>, grid, dim3(MCfg::NT), smem, s->stream, a));
     s->launches++;
@@ -545,12 +542,8 @@ int launch_indicator(fin_mhd* s, int buf)
     ia.zthr = s->zthr;
     ia.flags = s->flags;
     ia.count = s->ind_count;
-    static bool configured = false;
     const size_t smem = sizeof(MhdIndTile<ICfg>);
-    if (!configured) {
-        MCK(cudaFuncSetAttribute(k_mhd_indicator<ICfg>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-        configured = true;
-    }
+    MCK(s->smem.allow(k_mhd_indicator<ICfg>, smem));
     MCK(cudaMemsetAsync(s->flags, 0, flag_words(s->p.mx, s->p.my) * sizeof(unsigned), s->stream));
     const long long tiles = (long long)((s->p.mx + ICfg::TI - 1) / ICfg::TI) * ((s->p.my + ICfg::TJ - 1) / ICfg::TJ);
     const int grid = int(tiles < 148 * 3 ? tiles : 148 * 3);

@@ -23,6 +23,7 @@
 #include "fin_hybrid.cuh"
 #include "fin_tmap.h"
 #include "fin_pdl.h"
+#include "fin_smem.h"
 #include "fin_hostio.h"
 #include "fin_output.h"
 #include "fin_mpp.cuh"
@@ -99,6 +100,7 @@ struct fin_solver {
     double* d_face_x;       // per-face alpha buffers (only for fin_construct_l)
     double* d_face_y;
     cudaStream_t stream;
+    SmemGrants smem;
     cudaEvent_t ev0, ev1;
     cudaEvent_t kev[6];     // start/stop of the three stage kernels of the last step
     cudaEvent_t iev[2];     // start/stop of the indicator launch of the last step
@@ -406,11 +408,7 @@ int launch_stage_cfg(fin_solver* s, const StageArgs& a)
 {
     const size_t smem = Cfg::template smem_bytes<R>();
     auto kern = k_stage<R, VER, P2, Cfg, FG>;
-    static bool configured = false;   // per instantiation; attribute is per device function
-    if (!configured) {
-        CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-        configured = true;
-    }
+    CK(s->smem.allow(kern, smem));
     dim3 grid((a.my + Cfg::TJ - 1) / Cfg::TJ, (a.mx + Cfg::TI - 1) / Cfg::TI);
     CK(launch_pdl(kern, grid, dim3(Cfg::NT), smem, s->stream, a));
     s->launches++;
@@ -471,11 +469,7 @@ int launch_stage_hyb_t(fin_solver* s, const StageArgs& a)
 {
     using Lh = HybSmem<HybCfg>;
     auto kern = k_stage_hyb<VER, P2, HybCfg>;
-    static bool configured = false;   // per instantiation
-    if (!configured) {
-        CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(Lh::BYTES)));
-        configured = true;
-    }
+    CK(s->smem.allow(kern, Lh::BYTES));
     StageArgs b = a;
     b.tma = 0;
     const double* ext = (a.A && a.A != a.qin) ? a.A : ((a.B && a.B != a.qin) ? a.B : nullptr);
@@ -507,7 +501,8 @@ int launch_stage_hyb(fin_solver* s, const StageArgs& a)
 int launch_stage_hi(fin_solver* s, const StageArgs& a)
 {
     if (!fin::hi::built(s->p.space_order)) return set_err(FIN_ERR_ARG, "Requested WENO Reconstruction not implemented.");
-    CK(fin::hi::launch(s->p.space_order, s->p.weno_version, s->p.power_param == 2.0, a, s->stream));
+    CK(fin::hi::launch(s->p.space_order, s->p.weno_version, s->p.power_param == 2.0, a, s->smem,
+                       s->stream));
     s->launches++;
     return FIN_OK;
 }
@@ -717,12 +712,8 @@ int launch_indicator(fin_solver* s, int buf)
         ia.tma = 1;
         ia.tm = s->tm_q[buf];
     }
-    static bool configured = false;
     const size_t smem = sizeof(IndTile<Cfg>);
-    if (!configured) {
-        CK(cudaFuncSetAttribute(k_indicator<Cfg>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-        configured = true;
-    }
+    CK(s->smem.allow(k_indicator<Cfg>, smem));
     CK(cudaMemsetAsync(s->ind_count, 0, sizeof(unsigned long long), s->stream));
     CK(cudaMemsetAsync(s->flags, 0, flag_words(s->p.mx, s->p.my) * sizeof(unsigned), s->stream));
     const long long nf = (long long)(s->p.mx + 1) * s->p.my + (long long)s->p.mx * (s->p.my + 1);
