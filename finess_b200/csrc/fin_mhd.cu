@@ -9,7 +9,6 @@
 // slots and a stream.  Each stage is one launch of k_mhd_stage (fin_mhd.cuh);
 // per step the host reads back the face-speed maxima and the status word.
 #include <cuda_runtime.h>
-#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -22,6 +21,7 @@
 #include "fin_mhd_hyb.cuh"
 #include "fin_pdl.h"
 #include "fin_smem.h"
+#include "fin_wait.h"
 
 using namespace fin;
 
@@ -436,18 +436,9 @@ int read_step(fin_mhd* s, unsigned* st)
     const unsigned long long seq = ++s->seq;
     MCK(launch_pdl(k_mhd_publish, dim3(1), dim3(32), 0, s->stream, (const double*)s->slots, s->h_slots, seq));
     s->launches++;
-    const volatile unsigned long long* got = reinterpret_cast<volatile unsigned long long*>(s->h_slots + MS_SEQ);
-    for (unsigned n = 1; *got != seq; n++) {
-        if (n % 65536 == 0) {   // the stream stopped without the number: its error, if the number still is not there
-            const cudaError_t e = cudaStreamQuery(s->stream);
-            if (e != cudaErrorNotReady && *got != seq) {
-                MCK(e);
-                MCK(cudaStreamSynchronize(s->stream));
-                if (*got != seq) return merr(FIN_ERR_CUDA, "a step ended without its result");
-            }
-        }
-    }
-    std::atomic_thread_fence(std::memory_order_acquire);
+    bool there = false;
+    MCK(wait_number(reinterpret_cast<volatile unsigned long long*>(s->h_slots + MS_SEQ), seq, s->stream, &there));
+    if (!there) return merr(FIN_ERR_CUDA, "a step ended without its result");
     if (s->time_kernels) MCK(cudaStreamSynchronize(s->stream));   // the stages' events
     memcpy(st, s->h_slots + MS_STATUS, sizeof(*st));
     return FIN_OK;

@@ -12,7 +12,6 @@
 #include <cstdlib>
 #include <cstring>
 #include <cmath>
-#include <atomic>
 #include <string>
 #include <vector>
 #include <algorithm>
@@ -24,6 +23,7 @@
 #include "fin_tmap.h"
 #include "fin_pdl.h"
 #include "fin_smem.h"
+#include "fin_wait.h"
 #include "fin_hostio.h"
 #include "fin_output.h"
 #include "fin_mpp.cuh"
@@ -617,18 +617,9 @@ int finish_step(fin_solver* s)
                   s->slots + BLOCK * z, s->h_slots, seq));
     s->launches++;
     s->zb = z;
-    const volatile unsigned long long* got = reinterpret_cast<volatile unsigned long long*>(s->h_slots + SLOT_SEQ);
-    for (unsigned n = 1; *got != seq; n++) {
-        if (n % 65536 == 0) {   // the stream stopped without the number: its error, if the number still is not there
-            const cudaError_t e = cudaStreamQuery(s->stream);
-            if (e != cudaErrorNotReady && *got != seq) {
-                CK(e);
-                CK(cudaStreamSynchronize(s->stream));
-                if (*got != seq) return set_err(FIN_ERR_CUDA, "a step ended without its result");
-            }
-        }
-    }
-    std::atomic_thread_fence(std::memory_order_acquire);
+    bool there = false;
+    CK(wait_number(reinterpret_cast<volatile unsigned long long*>(s->h_slots + SLOT_SEQ), seq, s->stream, &there));
+    if (!there) return set_err(FIN_ERR_CUDA, "a step ended without its result");
     if (s->time_kernels) CK(cudaStreamSynchronize(s->stream));   // the stages' events
     return FIN_OK;
 }
