@@ -156,9 +156,11 @@ __global__ void k_mhd_publish(const double* slots, double* host, unsigned long l
     asm volatile("griddepcontrol.wait;" ::: "memory");
     static_assert(MS_N <= 32, "a lane a slot");
     if (threadIdx.x < MS_N) *const_cast<volatile double*>(host + threadIdx.x) = slots[threadIdx.x];
-    __threadfence_system();
-    __syncwarp();
-    if (threadIdx.x == 0) *reinterpret_cast<volatile unsigned long long*>(host + MS_SEQ) = seq;
+    __syncwarp();   // lane 0 has the other lanes' stores behind it, and its fence makes them all precede the number
+    if (threadIdx.x == 0) {
+        __threadfence_system();
+        *reinterpret_cast<volatile unsigned long long*>(host + MS_SEQ) = seq;
+    }
 }
 
 __global__ void k_mhd_state_max(const double* q, int mx, int my, size_t plane, double gamma, double* alpha_out,

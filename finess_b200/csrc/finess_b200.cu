@@ -247,9 +247,11 @@ __global__ void k_publish(const double* blk, const double* fixed, const double* 
         if (c == 0 || c == 1) v = alpha_cur[c];
         *const_cast<volatile double*>(host + k) = v;
     }
-    __threadfence_system();
-    __syncwarp();
-    if (k == 0) *reinterpret_cast<volatile unsigned long long*>(host + SLOT_SEQ) = seq;
+    __syncwarp();   // lane 0 has the other lanes' stores behind it, and its fence makes them all precede the number
+    if (k == 0) {
+        __threadfence_system();
+        *reinterpret_cast<volatile unsigned long long*>(host + SLOT_SEQ) = seq;
+    }
 }
 
 // max |a - b| and max |b| over all planes' interior values (judge step).

@@ -33,3 +33,21 @@ def test_many_small_steps(oracle, mx, my, method, time_order, mpp):
     qo = oracle.finsolve(p, q, 0.0, n * dt, dt)[1]
     assert all(np.array_equal(got[0], g) for g in got[1:])
     assert rel_linf(interior(p, got[0]), interior(p, qo)) <= 1e-11
+
+
+def test_published_maxima_repeat():
+    """The maxima that a step's last kernel hands to the host belong to that step:
+    the CFL numbers of many short steps repeat bit for bit."""
+    from finess_b200.mhd import MhdSolver
+    from finess_b200.solver import Solver
+    p, pm = P.vortex_params(n=24), P.orszag_tang_params(n=24)
+    q = P.random_smooth_state(p, np.random.default_rng(3))
+    m = P.mhd_random_state(pm, np.random.default_rng(3))
+    with Solver(p) as s, MhdSolver(pm) as h:
+        runs = []
+        for _ in range(4):
+            s.set_state(q)
+            h.set_state(*m)
+            runs.append([(s.step_fixed(1e-3), h.step_fixed(1e-3)) for _ in range(400)])
+    assert len(set(a for a, _ in runs[0])) > 300      # every step has maxima of its own
+    assert all(r == runs[0] for r in runs[1:])
