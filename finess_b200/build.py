@@ -20,6 +20,10 @@ NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-Xcompiler", "-fPIC",
     "-Xptxas", "-v",
+    # nvcc compresses a source's device code once it passes some size, and the
+    # first launch of a process then waits for the unpacking (first call of a
+    # process 15 ms, 7 without)
+    "-no-compress",
 ]
 SOURCES = ["finess_b200.cu", "fin_hi.cu", "fin_ini.cpp", "fin_noalloc.cu", "fin_mlp.cu", "fin_batch.cu", "fin_mhd.cu",
            "fin_output.cu"]
