@@ -432,7 +432,7 @@ k_stage_batch(const BProb* pr, const int* act, const long long* tile0, const int
 // k_stage_hyb; tiles of problems with tensor maps are staged by TMA on the
 // successive phases of one mbarrier).
 template <int VER, bool P2, class Cfg>
-__global__ void __launch_bounds__(Cfg::NT, FIN_HYB_CTAS)
+__global__ void __launch_bounds__(Cfg::NT, HYB_CTAS)
 k_stage_hyb_batch(const BProb* pr, const int* act, const long long* tile0, const int* nact, const StageArgs* args,
                   unsigned long long* queue)
 {

@@ -102,7 +102,6 @@ struct StageArgs {
     int tma;
     CUtensorMap tm_in;
     CUtensorMap tm_A;
-    CUtensorMap tm_qi;   // q_in with the interior-tile box (TJ x TI x 5)
     // The same two maps held in global memory (batches, whose stage
     // arguments live in global memory): used instead of tm_in / tm_A when
     // set, after a tensormap-proxy acquire fence.
@@ -166,12 +165,10 @@ struct TileCfg {
     static constexpr int FXR = TI + 3, FXC = TJ + 2, FYR = TI + 2, FYC = TJ + 3;
     static constexpr bool MASKS_FIT = FYC <= 32;   // flag row masks are 32-bit words
     // The FP64 staging tile of q_in (rows i0-3 .. i0+TI+2, columns j0-4 ..
-    // j0+TJ+3, so the TMA box starts on a 16-byte boundary) and the interior
-    // tile of a stage operand; a TMA destination starts on a 128-byte
-    // boundary, so buffers are padded to multiples of 128 bytes.
+    // j0+TJ+3, so the TMA box starts on a 16-byte boundary); a TMA destination
+    // starts on a 128-byte boundary, so offsets are padded to multiples of 128.
     static constexpr int SJ = TJ + 8;
     static constexpr size_t STG_BYTES = size_t(MEQN) * RI * SJ * 8;
-    static constexpr size_t ABUF_BYTES = size_t(MEQN) * TI * TJ * 8;
     __host__ __device__ static constexpr size_t pad128(size_t b) { return (b + 127) / 128 * 128; }
 };
 

@@ -13,8 +13,7 @@
 //     time and the speed computed twice (spills 118 -> 8 bytes a thread, and
 //     one-instruction maxima).
 // Layout and schedule, for B200:
-//   * one TI x TJ tile per CTA, four CTAs (32 warps) per SM (three: 30.7 ->
-//     32.2 ms for the steps above);
+//   * one TI x TJ tile per CTA, four CTAs (32 warps) per SM;
 //   * q_in's tile + halo arrives by one TMA copy (tiles clear of the domain
 //     boundary) into an FP64 staging tile, whose space the face fluxes take
 //     afterwards; the update reads both stage operands from L2, the one that is
@@ -32,21 +31,17 @@ namespace fin {
 
 using HybCfg = TileCfg<15, 16, 256>;
 
-// Resident CTAs per SM the kernel is laid out for: 3 keeps the update's
-// stage operands in shared memory (q_in's interior in the staging tile, the
-// other operand by a second TMA copy); 4 shares the staging tile's space with
-// the face fluxes and reads both operands from L2 (q_in's interior is there
-// from the tile's own copy, the other operand is prefetched into L2 by TMA),
-// within 64 registers a thread.
-#ifndef FIN_HYB_CTAS
-#define FIN_HYB_CTAS 4
-#endif
+// Resident CTAs per SM: the face fluxes share the staging tile's space, and the
+// update reads both stage operands from L2 (q_in's interior is there from the
+// tile's own copy, the other operand is prefetched into L2 by TMA), within 64
+// registers a thread.  With three, which leaves room for both operands in shared
+// memory, the steps above take 32.2 instead of 30.7 ms.
+constexpr int HYB_CTAS = 4;
 
 // Shared-memory layout (byte offsets) of k_stage_hyb.
 template <class Cfg>
 struct HybSmem {
     static constexpr int TI = Cfg::TI, TJ = Cfg::TJ, RI = Cfg::RI, RJ = Cfg::RJ, NT = Cfg::NT;
-    static constexpr bool SHARE = FIN_HYB_CTAS >= 4;
     static constexpr size_t PRIM = 0;                                                    // float4 [RI][RJ]
     static constexpr size_t FQX = PRIM + size_t(RI) * RJ * 16;                          // float2 [M][RI][TJ]
     static constexpr size_t FQY = FQX + size_t(MEQN) * RI * TJ * 8;                     // float2 [M][TI][RJ]
@@ -56,43 +51,25 @@ struct HybSmem {
     static constexpr int FP = TJ + 2;
     static constexpr size_t FHGH = size_t(MEQN) * ((TI + 1) + TI) * FP * 4;             // Fh, Gh bytes
     static constexpr size_t STG = Cfg::pad128(FQY + size_t(MEQN) * TI * RJ * 8);        // double [M][RI][SJ]
-    static constexpr size_t FH = SHARE ? STG : STG + Cfg::pad128(Cfg::STG_BYTES);       // float [M][TI+1][FP]
+    static constexpr size_t FH = STG;                                                   // float [M][TI+1][FP]
     static constexpr size_t GH = FH + size_t(MEQN) * (TI + 1) * FP * 4;                 // float [M][TI][FP]
-    static constexpr size_t EBUF = Cfg::pad128(SHARE ? STG + Cfg::STG_BYTES : FH + FHGH);   // double [M][TI][TJ]
-    static constexpr size_t RED = SHARE ? EBUF : EBUF + Cfg::ABUF_BYTES;               // double [NT/32][4]
+    static constexpr size_t RED = Cfg::pad128(STG + Cfg::STG_BYTES);                    // double [NT/32][4]
     static constexpr size_t MASK = RED + size_t(NT / 32) * 4 * 8;                       // unsigned [FXR + FYR]
     static constexpr size_t NTRB = MASK + 4 * size_t(Cfg::FXR + Cfg::FYR);              // int [2]
     static constexpr size_t TLIST = NTRB + 8;                                            // short [NFX + NFY]
     static constexpr size_t MBAR = (TLIST + 2 * size_t(Cfg::NFX + Cfg::NFY) + 7) / 8 * 8;   // uint64
     static constexpr size_t BYTES = MBAR + 8;
-    static_assert(!SHARE || FHGH <= Cfg::STG_BYTES, "the face fluxes fit the staging tile");
+    static_assert(FHGH <= Cfg::STG_BYTES, "the face fluxes fit the staging tile");
 };
 
-// linear_face on (0.5 f, q) pairs: P points at stencil point 3.  The f sums
-// and q differences run as f32x2 pairs, lane by lane the operations of
-//   sf = 37 (f2 + f3) + (-8 (f1 + f4) + (f0 + f5)),
-//   sq = 10 (q2 - q3) + (-5 (q1 - q4) + (q0 - q5)),
-// (x + y and x - y as fma(y, +-1, x): the same rounding).
-// The f32x2 form measured 1 % slower than the scalar one (B200, 4096^2,
-// mid-run state), so the scalar form is built.
-#ifndef FIN_X2_LINEAR
-#define FIN_X2_LINEAR 0
-#endif
+// linear_face on (0.5 f, q) pairs: P points at stencil point 3.  (With the f
+// sums and q differences as f32x2 pairs 1 % slower: B200, 4096^2, mid-run state.)
 __device__ __forceinline__ float linear_face2(const float2* P, int str, float lah)
 {
-#if FIN_X2_LINEAR
-    const f2 pm = f2_make(1.0f, -1.0f), k1 = f2_make(-8.0f, -5.0f), k2 = f2_make(37.0f, 10.0f);
-    const f2 s05 = f2_fma(f2_of(P[2 * str]), pm, f2_of(P[-3 * str]));
-    const f2 s14 = f2_fma(f2_of(P[str]), pm, f2_of(P[-2 * str]));
-    const f2 s23 = f2_fma(f2_of(P[0]), pm, f2_of(P[-str]));
-    const f2 t = f2_fma(k2, s23, f2_fma(k1, s14, s05));
-    return fmaf(lah, f2_hi(t), f2_lo(t)) * float(1.0 / 30.0);
-#else
     const float2 a0 = P[-3 * str], a1 = P[-2 * str], a2 = P[-str], a3 = P[0], a4 = P[str], a5 = P[2 * str];
     const float sf = fmaf(37.0f, a2.x + a3.x, fmaf(-8.0f, a1.x + a4.x, a0.x + a5.x));
     const float sq = fmaf(10.0f, a2.y - a3.y, fmaf(-5.0f, a1.y - a4.y, a0.y - a5.y));
     return fmaf(lah, sq, sf) * float(1.0 / 30.0);
-#endif
 }
 
 // Pass B of k_stage_hyb for one troubled face of direction x (ISX) or y, w
@@ -164,7 +141,7 @@ __device__ __forceinline__ void stage_hyb_tile(const StageArgs& a, const int i0,
     using L = HybSmem<Cfg>;
     static_assert(Cfg::MASKS_FIT, "flag row masks are 32-bit words");
     constexpr int TI = Cfg::TI, TJ = Cfg::TJ, NT = Cfg::NT, H = Cfg::H, RI = Cfg::RI, RJ = Cfg::RJ;
-    constexpr int XPL = RI * TJ, YPL = TI * RJ, TT = TI * TJ;   // component planes of fqx, fqy, ebuf
+    constexpr int XPL = RI * TJ, YPL = TI * RJ, TT = TI * TJ;   // component planes of fqx, fqy; cells
     constexpr int FP = L::FP;                                    // face-flux row pitch
     static_assert(TI == 15 && TJ == 16 && NT == 256 && NT >= TT, "one face / cell per thread, rows 8 apart");
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -179,7 +156,6 @@ __device__ __forceinline__ void stage_hyb_tile(const StageArgs& a, const int i0,
     int* ntrb = reinterpret_cast<int*>(smem_raw + L::NTRB);
     short* tlist = reinterpret_cast<short*>(smem_raw + L::TLIST);
     double* stg = reinterpret_cast<double*>(smem_raw + L::STG);
-    double* ebuf = reinterpret_cast<double*>(smem_raw + L::EBUF);   // the other operand's interior
     uint64_t* mbq = reinterpret_cast<uint64_t*>(smem_raw + L::MBAR);
 
     const int tid = threadIdx.x, lane = tid & 31;
@@ -188,22 +164,21 @@ __device__ __forceinline__ void stage_hyb_tile(const StageArgs& a, const int i0,
     const float ag1 = a.alpha_in ? float(a.alpha_in[0]) : 0.0f;
     const float ag2 = a.alpha_in ? float(a.alpha_in[1]) : 0.0f;
     const double* ext = (a.A && a.A != a.qin) ? a.A : ((a.B && a.B != a.qin) ? a.B : nullptr);
-    const bool aligned = ((tc::smem_addr(stg) | (L::SHARE ? 0u : tc::smem_addr(ebuf))) & 127u) == 0;
+    const bool aligned = (tc::smem_addr(stg) & 127u) == 0;
     if (a.tma && !aligned && tid == 0) atomicOr(a.status, 16u);
     const bool tt = a.tma && aligned && tma_interior<Cfg>(i0, j0, mx, my);
     float smax_x = 0.0f, smax_y = 0.0f, csx = 0.0f, csy = 0.0f;
     bool neg = false, nonfinite = false;
-    // ---- phase 0: q_in's tile + halo and the other operand's interior by
-    // TMA (or q_in through the boundary remap); the flag masks ----
+    // ---- phase 0: q_in's tile + halo by TMA (or through the boundary remap),
+    // the other operand's interior into L2; the flag masks ----
     if (tt && tid == 0) {
         const CUtensorMap* tmi = a.gtm_in ? a.gtm_in : &a.tm_in;
         const CUtensorMap* tme = a.gtm_A ? a.gtm_A : &a.tm_A;
         if (a.gtm_in) tc::tensormap_acquire(a.gtm_in);
         if (ext && a.gtm_A) tc::tensormap_acquire(a.gtm_A);
-        tc::mbar_expect_tx(mbq, uint32_t(Cfg::STG_BYTES + (ext && !L::SHARE ? Cfg::ABUF_BYTES : 0)));
+        tc::mbar_expect_tx(mbq, uint32_t(Cfg::STG_BYTES));
         tc::tma_load_3d(stg, tmi, j0 - 4, i0 - H, 0, mbq);
-        if (ext && !L::SHARE) tc::tma_load_3d(ebuf, tme, j0, i0, 0, mbq);
-        if (ext && L::SHARE) tc::tma_prefetch_3d(tme, j0, i0, 0);
+        if (ext) tc::tma_prefetch_3d(tme, j0, i0, 0);
     }
     {
         const int wx = flag_wx(my), wy = flag_wy(my);
@@ -386,8 +361,6 @@ __device__ __forceinline__ void stage_hyb_tile(const StageArgs& a, const int i0,
                 const size_t g = size_t(gi) * my + gj;
                 const float* fh = Fh + ci * FP + cj;
                 const float* gh = Gh + ci * FP + cj;
-                const double* si = stg + (H + ci) * Cfg::SJ + H + cj + 1;
-                const double* se = ebuf + ci * TJ + cj;
                 const double* ge = ext ? ext + g : nullptr;
                 double* out = a.qout + g;
                 // every operand load ahead of the first store: out may alias
@@ -396,8 +369,8 @@ __device__ __forceinline__ void stage_hyb_tile(const StageArgs& a, const int i0,
                 double qiv[MEQN], qev[MEQN];
 #pragma unroll
                 for (int m = 0; m < MEQN; m++) {
-                    qiv[m] = L::SHARE ? a.qin[m * plane + g] : si[m * RI * Cfg::SJ];
-                    qev[m] = (tt && !L::SHARE) ? se[m * TT] : (ge ? ge[m * plane] : 0.0);
+                    qiv[m] = a.qin[m * plane + g];
+                    qev[m] = ge ? ge[m * plane] : 0.0;
                 }
                 float qf[MEQN];
 #pragma unroll
@@ -450,7 +423,7 @@ __device__ __forceinline__ void stage_hyb_tile(const StageArgs& a, const int i0,
 
 // One CTA per tile of the state.
 template <int VER, bool P2, class Cfg>
-__global__ void __launch_bounds__(Cfg::NT, FIN_HYB_CTAS) k_stage_hyb(const __grid_constant__ StageArgs a)
+__global__ void __launch_bounds__(Cfg::NT, HYB_CTAS) k_stage_hyb(const __grid_constant__ StageArgs a)
 {
     const int ntj = (a.my + Cfg::TJ - 1) / Cfg::TJ;
     const int t = blockIdx.x;
