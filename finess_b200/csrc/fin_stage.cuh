@@ -232,13 +232,10 @@ __device__ __forceinline__ R linear_face(const R* f, int fstr, const R* q, int q
     return fma(lah, sq, sf) * R(1.0 / 30.0);
 }
 
-// Resident blocks per SM the register budget is sized for: FP64 faces need
-// about 110 registers a thread, FP32 about 70.
-// Measured on B200 at 4096^2 (stage-kernel ms, FP64 / FP32): one block per
-// SM 5.81 / 2.71; two FP64 blocks (128 registers, ~200 B spilled to L1) and
-// three FP32 blocks 4.07 / 2.44.  More resident warps beat the spills, up to
-// a point: four FP32 blocks (64 registers, 236 B spilled) took 2.14 ms where
-// three took 2.06 (the current kernel).
+// Resident blocks per SM the register budget is sized for.  Measured on B200 at
+// 4096^2, WENO5-Z, ms a stage: FP64 one block (164 registers) 3.33, two (122, no
+// spills) 2.39; FP32 two blocks (100 registers) 1.61, three (80, no spills) 1.281,
+// four (64, 20 bytes spilled) 1.285.
 #ifndef FIN_MINB_F64
 #define FIN_MINB_F64 2
 #endif

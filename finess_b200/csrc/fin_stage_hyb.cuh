@@ -8,7 +8,7 @@
 //   * troubled faces: the full characteristic WENO flux (weno_char_flux), x
 //     and y faces from lists of their own, so that every stencil address is a
 //     constant offset; pass A leaves each face's speed in its flux slot.
-//     Measured (B200, eight steps at 4096^2 with a third of the faces
+//     Measured (B200, eight steps at 4096^2 with 40 % of the faces
 //     troubled): 35.1 -> 31.0 ms against one list with strides chosen at run
 //     time and the speed computed twice (spills 118 -> 8 bytes a thread, and
 //     one-instruction maxima).

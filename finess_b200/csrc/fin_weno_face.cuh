@@ -31,7 +31,7 @@ __device__ __forceinline__ void wfence(float& x) { asm volatile("" : "+f"(x)); }
 // when the splits were projected point by point.  Fields 0, 4 and 1 in one
 // sweep, 2 and 3 in another: all five hold more registers than three or four
 // CTAs per SM leave.  Measured (B200): the FP32 stage, two steps of 4001 x
-// 515, 1.48 -> 1.16 ms; the hybrid form, eight steps at 4096^2 with a third
+// 515, 1.48 -> 1.16 ms; the hybrid form, eight steps at 4096^2 with 40 %
 // of the faces troubled, 40.0 -> 35.1 ms.
 template <int VER, bool P2, class Pt, class Park, class Parked>
 __device__ __forceinline__ void weno_char_flux(const Euler::Face<float>& ev, float lah, float eps, float pw, const Pt& pt,

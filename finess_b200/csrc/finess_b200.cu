@@ -420,9 +420,11 @@ int launch_stage_cfg(fin_solver* s, const StageArgs& a)
 // Grids of few tiles of 15 x 16 leave SMs idle or give some of them twice the
 // work of others: tiles of 7 x 16 with a thread for every face (one round instead
 // of two) spread them.  Twenty steps, us, 15 x 16 / 7 x 16:
-//   FP64 (with five memsets and a copy a step), up to SMALL64 tiles: 64^2 980 /
-//   872, 128^2 990 / 953, 160^2 1002 / 1002, 200^2 (182 tiles) 1249 / 1206; from
-//   256^2 (288) on the larger tile wins, 1260 / 1443;
+//   FP64 up to SMALL64 tiles of 15 x 16, 12 x 11 tiles 772 / 692, 13 x 12 980 /
+//   850, 15 x 13 (195) 992 / 900 (but 13 x 11, which have an SM each as they are,
+//   766 / 834); from 15 x 14 (210) on, where the smaller tiles
+//   are more than three an SM, the larger one wins, 986 / 1012, at 18 x 16 (288)
+//   992 / 1190;
 //   FP32, whose tile is shorter against the launch, while twice the tiles are at
 //   most one an SM: 32^2 607 / 517, 112^2 (56) 604 / 526, 128^2 (72) 607 / 572;
 //   144^2 (90) 607 / 604, 176^2 606 / 656, 320^2 918 / 1076.
@@ -1432,9 +1434,11 @@ int fin_construct_l(fin_solver* s, const double* q_host, double* L_host, double*
 // from the per-face speeds, then the status word.  Both are laid out on the
 // device, so the host moves whole rows: L's packed cells go to q[buf] (the input
 // state, read by now, of the same size), smax to the staging buffer.  300 x 257
-// with both: 1650 -> 740 us (a first call on a solver 4.3 -> 2.6 ms), 1000 x
-// 1100: 35 -> 12 ms (planes copied into a zeroed vector and transposed by the
-// host before).
+// with both: 1650 -> 740 us, 1000 x 1100: 35 -> 12 ms (planes copied into a zeroed
+// vector and transposed by the host before).  A solver's first call makes the
+// staging buffer, the face planes, the ring and its events: 4.5 -> 1.3 ms in a
+// process that has run one before, 9 and 10 to 13 in one that has not (loading the
+// kernels).
 static int download_l_smax(fin_solver* s, int buf, int outb, double* L_host, double* smax_host)
 {
     const fin_params& p = s->p;
